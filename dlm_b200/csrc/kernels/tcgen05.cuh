@@ -10,6 +10,7 @@ namespace dlmk {
 namespace tc5 {
 
 constexpr uint32_t WAIT_LIMIT = 1u << 22;       // try_wait calls before a wait gives up
+constexpr uint64_t WAIT_LIMIT_NS = 2000000000;  // nanoseconds before a wait gives up
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -30,11 +31,24 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return done != 0;
 }
-// Bounded wait.  Returns false when it gave up (or another role already had): the caller stops.
+__device__ __forceinline__ uint64_t global_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// Bounded wait.  Returns false when it gave up (or another role already had): the caller stops.  The bound is in time
+// (a try may itself block for a while, so a bound in tries alone could last minutes); the clock is read once every 16 tries,
+// which a wait that is met in time hardly ever reaches.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    uint64_t give_up = 0;
     for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
+        if ((i & 15) == 15) {
+            const uint64_t now = global_ns();
+            if (give_up == 0) give_up = now + WAIT_LIMIT_NS;
+            else if (now > give_up) break;
+        }
     }
     *abort_flag = 1;
     return false;
