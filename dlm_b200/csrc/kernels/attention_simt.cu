@@ -179,6 +179,12 @@ void attention_simt(const void* q, const void* k_cache, const void* v_cache, con
     if (T <= 0 || R <= 0) return;
     DLM_CHECK(hd > 0 && hd <= MAX_HD, "attention: head_dim must be in 1..256");
     DLM_CHECK(nh % nkv == 0, "attention: heads must be a multiple of kv heads");
+    if (dtype == F32 && attention_f32_ok(q, k_cache, v_cache, hd, scale)) {
+        attention_f32(static_cast<const float*>(q), static_cast<const float*>(k_cache), static_cast<const float*>(v_cache),
+                      block_table, table_width, cu_q, kv_len, static_cast<float*>(out), T, R, nh, nkv, hd, page_size,
+                      total_pages, window, scale, skip_single, stream);
+        return;
+    }
     const int tiles = (T + BQ - 1) / BQ + R;        // every request may end in a partial tile
     const size_t smem = sizeof(float) * (BQ * hd + BKV * (hd + 1) + BKV * hd + WARPS * QPW * BKV);
     dim3 grid(tiles, nh);
