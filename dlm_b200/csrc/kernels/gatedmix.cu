@@ -6,6 +6,7 @@
 // scans are.
 #include "api.h"
 #include "common.cuh"
+#include "scan_walk.h"
 
 namespace dlmk {
 namespace {
@@ -584,6 +585,19 @@ void gated_scan(const float* q, int ldq, const float* k, int ldk, const float* v
     DLM_CHECK(decay_kind == 0 || decay_kind == 1, "gated_scan: decay kind 0 (per head) or 1 (per key channel)");
     DLM_CHECK(decay_kind == 1 || A_log != nullptr, "gated_scan: a decay per head needs its rates");
     DLM_CHECK(decay_kind == 0 || tau > 0.f, "gated_scan: tau must be positive");
+    const bool delta = beta != nullptr && decay_kind == 0, channel = beta == nullptr && decay_kind == 1 && !unit;
+    if (delta || channel) {
+        WalkParams w{};
+        w.q = q; w.ldq = ldq; w.k = k; w.ldk = ldk; w.v = v; w.ldv = ldv; w.dec = dec; w.ldd = ldd;
+        w.beta = beta; w.ldb = ldb;
+        w.A_log = A_log; w.dec_bias = dec_bias;
+        w.state = state; w.cu_q = cu_q; w.state_slot = state_slot;
+        w.o = o; w.ldo = ldo;
+        w.heads = heads; w.q_div = heads / qk_heads; w.N = dk; w.P = dv;
+        w.unit = unit; w.unit_eps = unit_eps; w.q_scale = q_scale;
+        w.inv_tau = channel ? 1.0f / tau : 0.f;
+        if (scan_walk(delta ? WALK_DELTA : WALK_CHANNEL, w, R, stream)) return;
+    }
     launch_gated_scan(q, ldq, k, ldk, v, ldv, dec, ldd, beta, ldb, A_log, dec_bias, state, cu_q, state_slot, o, ldo, R,
                       heads, qk_heads, dk, dv, unit, unit_eps, q_scale, decay_kind, tau, MaxGateArgs{}, stream);
 }

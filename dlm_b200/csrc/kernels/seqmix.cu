@@ -8,6 +8,7 @@
 // own request only, in an order that does not depend on how the request was cut into steps.
 #include "api.h"
 #include "common.cuh"
+#include "scan_walk.h"
 
 namespace dlmk {
 namespace {
@@ -847,6 +848,19 @@ void ssm_scan(const float* xbc, int ldx, const float* dt_raw, int lddt, const fl
               "ssm_scan: without fixed decays the step sizes, their bias, A_log and D are needed");
     DLM_CHECK(groups >= 1 && heads % groups == 0, "ssm_scan: heads must be a multiple of groups");
     DLM_CHECK(N >= 1 && N <= 1024, "ssm_scan: state size 1..1024");
+    {
+        WalkParams w{};
+        w.q = xbc + (long long)heads * P + (long long)groups * N; w.ldq = ldx;
+        w.k = xbc + (long long)heads * P; w.ldk = ldx;
+        w.v = xbc; w.ldv = ldx;
+        w.dec = dt_raw; w.ldd = lddt;
+        w.A_log = A_log; w.dec_bias = dt_bias; w.D = D; w.fixed_decay = fixed_decay;
+        w.state = state; w.cu_q = cu_q; w.state_slot = state_slot;
+        w.o = y; w.ldo = heads * P;
+        w.heads = heads; w.q_div = heads / groups; w.N = N; w.P = P;
+        w.silu_inputs = silu_inputs;
+        if (scan_walk(WALK_HEAD, w, R, stream)) return;
+    }
     int parts, cols, chunks;
     const bool vec = N % 4 == 0;
     scan_layout(N, P, 8, &parts, &cols, &chunks, vec);   // few rows a lane: many lanes a column, many warps an SM
@@ -889,6 +903,19 @@ void delta_scan(const float* proj, int ld, int off_r, int off_k, int off_v, int 
                 int heads, int d, float unit_eps, float decay_coef, cudaStream_t stream) {
     if (R <= 0) return;
     DLM_CHECK(d >= 1 && d <= 512, "delta_scan: head size 1..512");
+    {
+        WalkParams w{};
+        w.q = proj + off_r; w.ldq = ld;
+        w.k = proj + off_k; w.ldk = ld;
+        w.v = proj + off_v; w.ldv = ld;
+        w.dec = lw; w.ldd = ldlw;
+        w.rate = proj + off_a; w.ldr = ld; w.rate_bias = a_bias;
+        w.state = state; w.cu_q = cu_q; w.state_slot = state_slot;
+        w.o = o; w.ldo = heads * d;
+        w.heads = heads; w.q_div = 1; w.N = d; w.P = d;
+        w.unit_eps = unit_eps; w.decay_coef = decay_coef;
+        if (scan_walk(WALK_REMOVE, w, R, stream)) return;
+    }
     int parts, cols, chunks;
     const bool vec = d % 4 == 0;
     scan_layout(d, d, 4, &parts, &cols, &chunks, vec);
