@@ -542,6 +542,257 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
     }
 }
 
+// The same for the tokens of a prompt: one block a run of 64 / HG tokens of a request and HG (8 or 16) of their heads, 64
+// rows of queries that meet every staged key row.  A token's own block (above) fetches its whole window for 16 rows, so
+// the fetch and the shared-memory reads of the keys bound it; here they are spent on four times the rows.  Per chunk of 32 keys:
+// scores S[64 x 32] over the row's k range in two halves (a warp: 32 rows x 16 keys x one half), the softmax step with four
+// threads a row (running maximum and sum in their registers), then O[64 x rank] += (P_hi + P_lo) C with a warp owning 8 NT
+// latent columns of all rows, its 16 NT accumulators in registers.  The next chunk's rows arrive meanwhile.
+constexpr int LR_ROWS = 64, LR_SP = LA_KC + 4;
+
+template <int NT, int HG>
+__global__ void __launch_bounds__(LA_THREADS, 1)
+latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_rot,
+                             const float* __restrict__ sink, const __nv_bfloat16* __restrict__ cache,
+                             const int32_t* __restrict__ block_table, int table_width, const int32_t* __restrict__ cu_q, int R,
+                             const int32_t* __restrict__ positions, __nv_bfloat16* lat, int Tn, int H, int dr, int rank,
+                             int page_size, int total_pages, int window, float scale, int* err) {
+    dep_wait();          // nothing is read or written before the kernels before this one have ended
+    typedef __nv_bfloat16 bf16;
+    constexpr int TB = LR_ROWS / HG;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_map[3];
+    const int width = rank + dr;
+    const int wk = (width + 63) & ~63;                      // k extent of the score product
+    const int qp = wk + 8;                                  // row pitch: 16 bytes off a multiple of 128
+    bf16* s_q = reinterpret_cast<bf16*>(smem_raw);          // [64][qp]
+    bf16* s_keys0 = s_q + (size_t)LR_ROWS * qp;             // [2][32][qp]
+    bf16* s_pb = s_keys0 + (size_t)2 * LA_KC * qp;          // [2][64][LM_PP] weights, high and low term
+    float* s_s = reinterpret_cast<float*>(s_pb + 2 * LR_ROWS * LM_PP);   // [2][64][LR_SP] scores of the two k halves
+    float* s_corr = s_s + 2 * LR_ROWS * LR_SP;              // [64]
+    float* s_m = s_corr + LR_ROWS;
+    float* s_l = s_m + LR_ROWS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, tq = lane & 3;
+    const int h0 = blockIdx.y * HG;
+    if (tid == 0) {                                         // late runs (most keys) first
+        const int want = (int)gridDim.x - 1 - (int)blockIdx.x;
+        int acc = 0;
+        s_map[0] = -1;
+        for (int r = 0; r < R; ++r) {
+            const int b = cu_q[r], e = cu_q[r + 1], runs = (e - b + TB - 1) / TB;
+            if (want < acc + runs) {
+                s_map[0] = r;
+                s_map[1] = b + (want - acc) * TB;
+                s_map[2] = min(TB, e - s_map[1]);
+                break;
+            }
+            acc += runs;
+        }
+    }
+    __syncthreads();
+    const int req = s_map[0];
+    if (req < 0) return;
+    const int t0 = s_map[1], n_tok = s_map[2];
+    // the rows, (token, head), as bfloat16; rows without a token or a head are zeros
+    for (int idx = tid; idx < LR_ROWS * (qp / 4); idx += LA_THREADS) {
+        const int row = idx / (qp / 4), c = 4 * (idx - row * (qp / 4));
+        const int i = row / HG, h = h0 + row % HG;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n_tok && h < H) {
+            if (c < rank) v = *reinterpret_cast<const float4*>(q_lat + ((long long)h * Tn + t0 + i) * rank + c);
+            else if (c < width) v = *reinterpret_cast<const float4*>(q_rot + ((long long)(t0 + i) * H + h) * dr + (c - rank));
+        }
+        *reinterpret_cast<uint2*>(s_q + (size_t)row * qp + c) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    }
+    for (int idx = tid; idx < 2 * LA_KC * (qp - width); idx += LA_THREADS) {     // the padding stays zero
+        const int row = idx / (qp - width), c = idx - row * (qp - width);
+        s_keys0[(size_t)row * qp + width + c] = __float2bfloat16_rn(0.f);
+    }
+    float acc[4][NT][4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f;
+
+    const int32_t* table = block_table + (long long)req * table_width;
+    const int p_first = positions[t0], p_last = positions[t0 + n_tok - 1];
+    const int lo = window > 0 ? max(p_first - window + 1, 0) : 0;
+    const int c_begin = lo / LA_KC, c_end = p_last / LA_KC + 1;
+    auto stage = [&](int ch, int which) {
+        bf16* base = s_keys0 + (size_t)which * LA_KC * qp;
+        for (int jj = warp; jj < LA_KC; jj += LA_THREADS / 32) {
+            const int j = ch * LA_KC + jj;
+            bf16* dst = base + (size_t)jj * qp;
+            const bf16* row = nullptr;
+            if (j >= lo && j <= p_last) {
+                const int lp = j / page_size;
+                const int page = lp < table_width ? table[lp] : -1;
+                if (page < 0 || page >= total_pages) {
+                    if (lane == 0) *err = 3;
+                } else {
+                    row = cache + ((long long)page * page_size + (j - lp * page_size)) * width;
+                }
+            }
+            if (row == nullptr) {
+                uint4* d4 = reinterpret_cast<uint4*>(dst);
+                for (int i = lane; i < width / 8; i += 32) d4[i] = make_uint4(0u, 0u, 0u, 0u);
+            } else {
+                for (int i = lane; i < width / 8; i += 32) cp_async16(dst + 8 * i, row + 8 * i);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the softmax's row of this thread
+    const int srow = tid >> 2, sub = tid & 3;
+    const int p_row = srow / HG < n_tok ? positions[t0 + srow / HG] : -1;
+    const int lo_row = window > 0 ? max(p_row - window + 1, 0) : 0;
+    float m_run = -INFINITY, l_run = 0.f;
+    const int arow = (lane & 7) + 8 * ((lane >> 3) & 1);    // the row a lane names in a 16-row ldmatrix.x4
+    const int n_base = warp * NT * 8;
+    const int mw = warp & 1, nw = (warp >> 1) & 1, kh = warp >> 2;
+    const int half = wk / 32;                               // k steps of 16 in a half
+
+    stage(c_begin, 0);
+    for (int ch = c_begin; ch < c_end; ++ch) {
+        const bf16* s_keys = s_keys0 + (size_t)((ch - c_begin) & 1) * LA_KC * qp;
+        __syncthreads();                                    // the chunk before is done with the other buffer and with s_pb
+        if (ch + 1 < c_end) {
+            stage(ch + 1, (ch + 1 - c_begin) & 1);          // the next chunk comes in while this one is worked on
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        {
+            float c[2][2][4];
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) c[m][n][0] = c[m][n][1] = c[m][n][2] = c[m][n][3] = 0.f;
+            const bf16* abase = s_q + (size_t)(32 * mw + arow) * qp + 8 * (lane >> 4) + kh * half * 16;
+            const bf16* bbase = s_keys + (size_t)(16 * nw + (lane & 7) + 8 * (lane >> 4)) * qp + 8 * ((lane >> 3) & 1) + kh * half * 16;
+#pragma unroll 3
+            for (int ks = 0; ks < half; ++ks) {
+                uint32_t a0[4], a1[4], b[4];
+                ldsm_x4(a0, abase + ks * 16);
+                ldsm_x4(a1, abase + (size_t)16 * qp + ks * 16);
+                ldsm_x4(b, bbase + ks * 16);                // keys 0-7 (two k halves), keys 8-15 (two k halves)
+                mma16816(c[0][0], a0, b[0], b[1]);
+                mma16816(c[0][1], a0, b[2], b[3]);
+                mma16816(c[1][0], a1, b[0], b[1]);
+                mma16816(c[1][1], a1, b[2], b[3]);
+            }
+            float* dst = s_s + (size_t)kh * LR_ROWS * LR_SP;
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    float* d = dst + (32 * mw + 16 * m + g) * LR_SP + 16 * nw + 8 * n + 2 * tq;
+                    *reinterpret_cast<float2*>(d) = make_float2(c[m][n][0], c[m][n][1]);
+                    *reinterpret_cast<float2*>(d + 8 * LR_SP) = make_float2(c[m][n][2], c[m][n][3]);
+                }
+        }
+        __syncthreads();
+        {
+            float sc[8];
+            const float* s0 = s_s + srow * LR_SP + 8 * sub;
+            const float* s1 = s0 + LR_ROWS * LR_SP;
+            float mx = -INFINITY;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int j = ch * LA_KC + 8 * sub + e;
+                sc[e] = (s0[e] + s1[e]) * scale;
+                if (j < lo_row || j > p_row) sc[e] = -INFINITY;
+                mx = fmaxf(mx, sc[e]);
+            }
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float m_new = fmaxf(m_run, mx);
+            float corr = 1.f, sum = 0.f;
+            uint32_t hi[4], lw[4];
+            if (m_new > -INFINITY) corr = expf(m_run - m_new);
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                const float pa = m_new > -INFINITY ? expf(sc[e] - m_new) : 0.f;
+                const float pb = m_new > -INFINITY ? expf(sc[e + 1] - m_new) : 0.f;
+                sum += pa + pb;
+                const bf16 ha = __float2bfloat16_rn(pa), hb = __float2bfloat16_rn(pb);
+                hi[e / 2] = pack_bf16(pa, pb);
+                lw[e / 2] = pack_bf16(pa - __bfloat162float(ha), pb - __bfloat162float(hb));
+            }
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            *reinterpret_cast<uint4*>(s_pb + srow * LM_PP + 8 * sub) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(s_pb + (LR_ROWS + srow) * LM_PP + 8 * sub) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+            l_run = l_run * corr + sum;
+            m_run = m_new;
+            if (sub == 0) s_corr[srow] = corr;
+        }
+        __syncthreads();
+        {
+            float c0[4], c1[4];
+            bool same = true;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                c0[m] = s_corr[16 * m + g];
+                c1[m] = s_corr[16 * m + g + 8];
+                same = same && c0[m] == 1.f && c1[m] == 1.f;
+            }
+            if (!__all_sync(0xffffffffu, same)) {           // the maxima move seldom once a row has seen some keys
+#pragma unroll
+                for (int m = 0; m < 4; ++m)
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        acc[m][n][0] *= c0[m]; acc[m][n][1] *= c0[m]; acc[m][n][2] *= c1[m]; acc[m][n][3] *= c1[m];
+                    }
+            }
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+                uint32_t b[NT / 2][4];
+                const bf16* kb = s_keys + (size_t)(kk * 16 + arow) * qp + n_base + 8 * (lane >> 4);
+#pragma unroll
+                for (int n = 0; n < NT; n += 2) ldsm_x4_trans(b[n / 2], kb + n * 8);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    uint32_t ah[4], al[4];
+                    const bf16* pa = s_pb + (16 * m + arow) * LM_PP + kk * 16 + 8 * (lane >> 4);
+                    ldsm_x4(ah, pa);
+                    ldsm_x4(al, pa + LR_ROWS * LM_PP);
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        mma16816(acc[m][n], ah, b[n / 2][2 * (n & 1)], b[n / 2][2 * (n & 1) + 1]);
+                        mma16816(acc[m][n], al, b[n / 2][2 * (n & 1)], b[n / 2][2 * (n & 1) + 1]);
+                    }
+                }
+            }
+        }
+    }
+    if (sub == 0) {
+        s_m[srow] = m_run;
+        s_l[srow] = l_run;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr) {
+            const int row = 16 * m + g + 8 * rr;
+            const int i = row / HG, h = h0 + row % HG;
+            if (i >= n_tok || h >= H) continue;
+            const float snk = sink ? sink[h] : -INFINITY;
+            const float mm = fmaxf(s_m[row], snk);
+            const float f = s_l[row] > 0.f ? expf(s_m[row] - mm) : 0.f;
+            const float den = s_l[row] * f + (sink ? expf(snk - mm) : 0.f);
+            const float w = den > 0.f ? f / den : 0.f;
+            bf16* dst = lat + ((long long)h * Tn + t0 + i) * rank;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+                *reinterpret_cast<uint32_t*>(dst + n_base + n * 8 + 2 * tq) =
+                    pack_bf16(acc[m][n][2 * rr] * w, acc[m][n][2 * rr + 1] * w);
+        }
+}
+
 // Merges the splits of a (token, head) in order and normalises as above.  One block a (token, head).
 template <typename T>
 __global__ void latent_merge_kernel(const float* __restrict__ partial, int n_splits, const float* __restrict__ sink,
@@ -635,8 +886,19 @@ bool latent_use_mma(int dtype, int rank, int dr, int fast) {
     return fast && !off && dtype == BF16 && rank % 128 == 0 && rank <= 512 && dr % 8 == 0;
 }
 
-int latent_attention_splits(int T, int H, int rank, int dr, int max_keys, int dtype, int fast) {
+namespace {
+int rows_heads(int H) { return H <= 8 ? 8 : 16; }           // heads a block of the many-row kernel takes
+// The many-row kernel: prompts (eight tokens a request and more) that give it a block for every other multiprocessor.
+bool latent_use_rows(int T, int R, int H, int rank, int dr, int dtype, int fast) {
+    const int hg = rows_heads(H);
+    return latent_use_mma(dtype, rank, dr, fast) && R > 0 && T >= 8 * R &&
+           (long long)(T / (LR_ROWS / hg)) * ((H + hg - 1) / hg) >= sm_count() / 2;
+}
+}  // namespace
+
+int latent_attention_splits(int T, int R, int H, int rank, int dr, int max_keys, int dtype, int fast) {
     if (dtype == F32 || T <= 0) return 1;       // 32-bit: one order of summation whatever the step holds
+    if (latent_use_rows(T, R, H, rank, dr, dtype, fast)) return 1;
     const int blocks = latent_use_mma(dtype, rank, dr, fast)
                            ? T * ((H + LM_ROWS - 1) / LM_ROWS)
                            : T * ((H + heads_per_block(H) - 1) / heads_per_block(H));
@@ -673,11 +935,38 @@ void latent_gate_out(const float* val, const float* gate, int ldg, void* out, in
 
 void latent_attention(const float* q_lat, const float* q_rot, const float* sink, const void* cache,
                       const int32_t* block_table, int table_width, const int32_t* token_req, const int32_t* positions,
-                      void* lat, float* partial, int n_splits, int T, int H, int dr, int rank, int page_size,
-                      int total_pages, int window, float scale, int dtype, int fast, cudaStream_t stream) {
+                      const int32_t* cu_q, int R, void* lat, float* partial, int n_splits, int T, int H, int dr, int rank,
+                      int page_size, int total_pages, int window, float scale, int dtype, int fast, cudaStream_t stream) {
     if (T <= 0) return;
     DLM_CHECK(rank >= 1 && rank <= 1024, "latent_attention: latent size 1..1024");
     DLM_CHECK(n_splits >= 1 && (n_splits == 1 || partial != nullptr), "latent_attention: splits need a scratch buffer");
+    if (n_splits == 1 && latent_use_rows(T, R, H, rank, dr, dtype, fast)) {
+        const int hg = rows_heads(H), tb = LR_ROWS / hg;
+        const int qp = ((rank + dr + 63) & ~63) + 8;
+        const size_t smem = ((size_t)(LR_ROWS + 2 * LA_KC) * qp + 2 * LR_ROWS * LM_PP) * sizeof(__nv_bfloat16) +
+                            (2 * LR_ROWS * LR_SP + 3 * LR_ROWS) * sizeof(float);
+        const dim3 grid(T / tb + R, (H + hg - 1) / hg);     // every request may end in a partial run
+#define DLM_LROWS(NT, HG)                                                                                             \
+    do {                                                                                                              \
+        auto kern = latent_attention_rows_kernel<NT, HG>;                                                             \
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
+        kern<<<grid, LA_THREADS, smem, stream>>>(q_lat, q_rot, sink, static_cast<const __nv_bfloat16*>(cache),        \
+                                                 block_table, table_width, cu_q, R, positions,                        \
+                                                 static_cast<__nv_bfloat16*>(lat), T, H, dr, rank, page_size,         \
+                                                 total_pages, window, scale, error_flag_ptr());                       \
+    } while (0)
+#define DLM_LROWS_H(NT) do { if (hg == 8) DLM_LROWS(NT, 8); else DLM_LROWS(NT, 16); } while (0)
+        switch (rank / 64) {
+            case 2: DLM_LROWS_H(2); break;
+            case 4: DLM_LROWS_H(4); break;
+            case 6: DLM_LROWS_H(6); break;
+            default: DLM_LROWS_H(8); break;
+        }
+#undef DLM_LROWS_H
+#undef DLM_LROWS
+        check_launch("latent_attention (rows)");
+        return;
+    }
     if (latent_use_mma(dtype, rank, dr, fast)) {
         const int wk = (rank + dr + 63) & ~63, qp = wk + 8;
         const size_t smem = ((size_t)(LM_ROWS + 2 * LA_KC) * qp + 2 * LM_ROWS * LM_PP) * sizeof(__nv_bfloat16) +
