@@ -82,7 +82,10 @@ def build_spec(cfg: ZasazenConfig) -> ModelSpec:
     return ModelSpec(hidden_size=cfg.width, vocab_size=cfg.vocab, layers=layers, layer_prefixes=prefixes,
                      final_norm=norm, final_norm_prefix="final.norm", embed_name="embed", lm_head_name="head",
                      embed_scale=cfg.embedding_scale, order=layer_order(len(cfg.layers), cfg.loop),
-                     pass_entry=entry, pass_entry_prefix="loop.")
+                     pass_entry=entry, pass_entry_prefix="loop.",
+                     # prompts have stopped answering now and then behind this design's sequence of launches (two of five
+                     # processes that ran other models before it), as another design's did until it took ordinary ones
+                     dependent_launch_tokens=64)
 
 
 register_architecture(ZasazenConfig.architecture, ZasazenConfig, build_spec, model_type=ZasazenConfig.model_type)

@@ -46,6 +46,7 @@ class ModelSpec:
     logit_softcap: float = 0.0               # c > 0: the logits are ``c tanh(head product / c)``
     dependent_launch: bool = True            # False: this model's steps launch every kernel in the ordinary way (each
                                              # starts when the one before it has ended) where the backend has the choice
+    dependent_launch_tokens: int | None = None   # the same for the steps of more than this many tokens
 
 
 class WeightError(ValueError):
@@ -181,7 +182,9 @@ class DecoderModel:
         """Runs the batch's tokens through every call of the order, reading and writing
         ``cache``; returns 32-bit logits ``[len(batch.logit_rows), vocab]``."""
         rt, ops = self.rt, self.rt.ops
-        if not self.spec.dependent_launch and hasattr(ops, "dependent_launch"):
+        most = self.spec.dependent_launch_tokens
+        off = not self.spec.dependent_launch or (most is not None and batch.num_tokens > most)
+        if off and hasattr(ops, "dependent_launch"):
             with ops.dependent_launch(False):
                 return self._step(batch, cache)
         return self._step(batch, cache)
