@@ -545,13 +545,15 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
 // The same for the tokens of a prompt: one block a run of 64 / HG tokens of a request and HG (8 or 16) of their heads, 64
 // rows of queries that meet every staged key row.  A token's own block (above) fetches its whole window for 16 rows, so
 // the fetch and the shared-memory reads of the keys bound it; here they are spent on four times the rows.  Per chunk of 32 keys:
-// scores S[64 x 32] over the row's k range in two halves (a warp: 32 rows x 16 keys x one half), the softmax step with four
+// scores S[64 x 32] over the row's k range in W / 4 parts (a warp: 32 rows x 16 keys x one part), the softmax step with W / 2
 // threads a row (running maximum and sum in their registers), then O[64 x rank] += (P_hi + P_lo) C with a warp owning 8 NT
-// latent columns of all rows, its 16 NT accumulators in registers.  The next chunk's rows arrive meanwhile.
+// latent columns of all rows, its 16 NT accumulators in registers.  The next chunk's rows arrive meanwhile.  The phases lie between
+// barriers, so what hides one warp's latency is the other warps: W = 16 where a warp's share of the latent is then a multiple of 16
+// columns (a rank of 256 or 512), else 8.
 constexpr int LR_ROWS = 64, LR_SP = LA_KC + 4;
 
-template <int NT, int HG>
-__global__ void __launch_bounds__(LA_THREADS, 1)
+template <int NT, int HG, int W>
+__global__ void __launch_bounds__(32 * W, 1)
 latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_rot,
                              const float* __restrict__ sink, const __nv_bfloat16* __restrict__ cache,
                              const int32_t* __restrict__ block_table, int table_width, const int32_t* __restrict__ cu_q, int R,
@@ -559,7 +561,7 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
                              int page_size, int total_pages, int window, float scale, int* err) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     typedef __nv_bfloat16 bf16;
-    constexpr int TB = LR_ROWS / HG;
+    constexpr int TB = LR_ROWS / HG, THREADS = 32 * W, KQ = W / 4, TPR = W / 2, KPT = LA_KC / TPR;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_map[3];
     const int width = rank + dr;
@@ -568,8 +570,8 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
     bf16* s_q = reinterpret_cast<bf16*>(smem_raw);          // [64][qp]
     bf16* s_keys0 = s_q + (size_t)LR_ROWS * qp;             // [2][32][qp]
     bf16* s_pb = s_keys0 + (size_t)2 * LA_KC * qp;          // [2][64][LM_PP] weights, high and low term
-    float* s_s = reinterpret_cast<float*>(s_pb + 2 * LR_ROWS * LM_PP);   // [2][64][LR_SP] scores of the two k halves
-    float* s_corr = s_s + 2 * LR_ROWS * LR_SP;              // [64]
+    float* s_s = reinterpret_cast<float*>(s_pb + 2 * LR_ROWS * LM_PP);   // [KQ][64][LR_SP] scores of the parts of k
+    float* s_corr = s_s + KQ * LR_ROWS * LR_SP;              // [64]
     float* s_m = s_corr + LR_ROWS;
     float* s_l = s_m + LR_ROWS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -595,7 +597,7 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
     if (req < 0) return;
     const int t0 = s_map[1], n_tok = s_map[2];
     // the rows, (token, head), as bfloat16; rows without a token or a head are zeros
-    for (int idx = tid; idx < LR_ROWS * (qp / 4); idx += LA_THREADS) {
+    for (int idx = tid; idx < LR_ROWS * (qp / 4); idx += THREADS) {
         const int row = idx / (qp / 4), c = 4 * (idx - row * (qp / 4));
         const int i = row / HG, h = h0 + row % HG;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -605,7 +607,7 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
         }
         *reinterpret_cast<uint2*>(s_q + (size_t)row * qp + c) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
     }
-    for (int idx = tid; idx < 2 * LA_KC * (qp - width); idx += LA_THREADS) {     // the padding stays zero
+    for (int idx = tid; idx < 2 * LA_KC * (qp - width); idx += THREADS) {     // the padding stays zero
         const int row = idx / (qp - width), c = idx - row * (qp - width);
         s_keys0[(size_t)row * qp + width + c] = __float2bfloat16_rn(0.f);
     }
@@ -621,7 +623,7 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
     const int c_begin = lo / LA_KC, c_end = p_last / LA_KC + 1;
     auto stage = [&](int ch, int which) {
         bf16* base = s_keys0 + (size_t)which * LA_KC * qp;
-        for (int jj = warp; jj < LA_KC; jj += LA_THREADS / 32) {
+        for (int jj = warp; jj < LA_KC; jj += W) {
             const int j = ch * LA_KC + jj;
             bf16* dst = base + (size_t)jj * qp;
             const bf16* row = nullptr;
@@ -644,14 +646,14 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     // the softmax's row of this thread
-    const int srow = tid >> 2, sub = tid & 3;
+    const int srow = tid / TPR, sub = tid % TPR;
     const int p_row = srow / HG < n_tok ? positions[t0 + srow / HG] : -1;
     const int lo_row = window > 0 ? max(p_row - window + 1, 0) : 0;
     float m_run = -INFINITY, l_run = 0.f;
     const int arow = (lane & 7) + 8 * ((lane >> 3) & 1);    // the row a lane names in a 16-row ldmatrix.x4
     const int n_base = warp * NT * 8;
     const int mw = warp & 1, nw = (warp >> 1) & 1, kh = warp >> 2;
-    const int half = wk / 32;                               // k steps of 16 in a half
+    const int half = wk / (16 * KQ);                        // k steps of 16 in a part (wk is a multiple of 64)
 
     stage(c_begin, 0);
     for (int ch = c_begin; ch < c_end; ++ch) {
@@ -695,25 +697,27 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
         }
         __syncthreads();
         {
-            float sc[8];
-            const float* s0 = s_s + srow * LR_SP + 8 * sub;
-            const float* s1 = s0 + LR_ROWS * LR_SP;
+            float sc[KPT];
+            const float* s0 = s_s + srow * LR_SP + KPT * sub;
             float mx = -INFINITY;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int j = ch * LA_KC + 8 * sub + e;
-                sc[e] = (s0[e] + s1[e]) * scale;
+            for (int e = 0; e < KPT; ++e) {
+                const int j = ch * LA_KC + KPT * sub + e;
+                float dot = s0[e];
+#pragma unroll
+                for (int part = 1; part < KQ; ++part) dot += s0[part * LR_ROWS * LR_SP + e];
+                sc[e] = dot * scale;
                 if (j < lo_row || j > p_row) sc[e] = -INFINITY;
                 mx = fmaxf(mx, sc[e]);
             }
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+#pragma unroll
+            for (int o = 1; o < TPR; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
             const float m_new = fmaxf(m_run, mx);
             float corr = 1.f, sum = 0.f;
-            uint32_t hi[4], lw[4];
+            uint32_t hi[KPT / 2], lw[KPT / 2];
             if (m_new > -INFINITY) corr = expf(m_run - m_new);
 #pragma unroll
-            for (int e = 0; e < 8; e += 2) {
+            for (int e = 0; e < KPT; e += 2) {
                 const float pa = m_new > -INFINITY ? expf(sc[e] - m_new) : 0.f;
                 const float pb = m_new > -INFINITY ? expf(sc[e + 1] - m_new) : 0.f;
                 sum += pa + pb;
@@ -721,10 +725,14 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
                 hi[e / 2] = pack_bf16(pa, pb);
                 lw[e / 2] = pack_bf16(pa - __bfloat162float(ha), pb - __bfloat162float(hb));
             }
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            *reinterpret_cast<uint4*>(s_pb + srow * LM_PP + 8 * sub) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(s_pb + (LR_ROWS + srow) * LM_PP + 8 * sub) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+#pragma unroll
+            for (int o = 1; o < TPR; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            bf16* dst = s_pb + srow * LM_PP + KPT * sub;
+#pragma unroll
+            for (int e = 0; e < KPT / 2; e += 2) {
+                *reinterpret_cast<uint2*>(dst + 2 * e) = make_uint2(hi[e], hi[e + 1]);
+                *reinterpret_cast<uint2*>(dst + LR_ROWS * LM_PP + 2 * e) = make_uint2(lw[e], lw[e + 1]);
+            }
             l_run = l_run * corr + sum;
             m_run = m_new;
             if (sub == 0) s_corr[srow] = corr;
@@ -888,10 +896,17 @@ bool latent_use_mma(int dtype, int rank, int dr, int fast) {
 
 namespace {
 int rows_heads(int H) { return H <= 8 ? 8 : 16; }           // heads a block of the many-row kernel takes
-// The many-row kernel: prompts (eight tokens a request and more) that give it a block for every other multiprocessor.
+int rows_warps(int rank) { return rank % 256 == 0 ? 16 : 8; }
+size_t rows_smem(int rank, int dr) {
+    const int qp = ((rank + dr + 63) & ~63) + 8;
+    return ((size_t)(LR_ROWS + 2 * LA_KC) * qp + 2 * LR_ROWS * LM_PP) * sizeof(__nv_bfloat16) +
+           (rows_warps(rank) / 4 * LR_ROWS * LR_SP + 3 * LR_ROWS) * sizeof(float);
+}
+// The many-row kernel: prompts (eight tokens a request and more) that give it a block for every other multiprocessor, and rows
+// of which 128 fit in shared memory.
 bool latent_use_rows(int T, int R, int H, int rank, int dr, int dtype, int fast) {
     const int hg = rows_heads(H);
-    return latent_use_mma(dtype, rank, dr, fast) && R > 0 && T >= 8 * R &&
+    return latent_use_mma(dtype, rank, dr, fast) && R > 0 && T >= 8 * R && rows_smem(rank, dr) <= 226 * 1024 &&
            (long long)(T / (LR_ROWS / hg)) * ((H + hg - 1) / hg) >= sm_count() / 2;
 }
 }  // namespace
@@ -942,25 +957,23 @@ void latent_attention(const float* q_lat, const float* q_rot, const float* sink,
     DLM_CHECK(n_splits >= 1 && (n_splits == 1 || partial != nullptr), "latent_attention: splits need a scratch buffer");
     if (n_splits == 1 && latent_use_rows(T, R, H, rank, dr, dtype, fast)) {
         const int hg = rows_heads(H), tb = LR_ROWS / hg;
-        const int qp = ((rank + dr + 63) & ~63) + 8;
-        const size_t smem = ((size_t)(LR_ROWS + 2 * LA_KC) * qp + 2 * LR_ROWS * LM_PP) * sizeof(__nv_bfloat16) +
-                            (2 * LR_ROWS * LR_SP + 3 * LR_ROWS) * sizeof(float);
+        const size_t smem = rows_smem(rank, dr);
         const dim3 grid(T / tb + R, (H + hg - 1) / hg);     // every request may end in a partial run
-#define DLM_LROWS(NT, HG)                                                                                             \
+#define DLM_LROWS(NT, HG, W)                                                                                          \
     do {                                                                                                              \
-        auto kern = latent_attention_rows_kernel<NT, HG>;                                                             \
+        auto kern = latent_attention_rows_kernel<NT, HG, W>;                                                          \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
-        kern<<<grid, LA_THREADS, smem, stream>>>(q_lat, q_rot, sink, static_cast<const __nv_bfloat16*>(cache),        \
-                                                 block_table, table_width, cu_q, R, positions,                        \
-                                                 static_cast<__nv_bfloat16*>(lat), T, H, dr, rank, page_size,         \
-                                                 total_pages, window, scale, error_flag_ptr());                       \
+        kern<<<grid, 32 * W, smem, stream>>>(q_lat, q_rot, sink, static_cast<const __nv_bfloat16*>(cache),            \
+                                             block_table, table_width, cu_q, R, positions,                            \
+                                             static_cast<__nv_bfloat16*>(lat), T, H, dr, rank, page_size,             \
+                                             total_pages, window, scale, error_flag_ptr());                           \
     } while (0)
-#define DLM_LROWS_H(NT) do { if (hg == 8) DLM_LROWS(NT, 8); else DLM_LROWS(NT, 16); } while (0)
-        switch (rank / 64) {
-            case 2: DLM_LROWS_H(2); break;
-            case 4: DLM_LROWS_H(4); break;
-            case 6: DLM_LROWS_H(6); break;
-            default: DLM_LROWS_H(8); break;
+#define DLM_LROWS_H(NT, W) do { if (hg == 8) DLM_LROWS(NT, 8, W); else DLM_LROWS(NT, 16, W); } while (0)
+        switch (rank / 64) {                                // NT = rank / (8 W), W = rows_warps(rank)
+            case 2: DLM_LROWS_H(2, 8); break;
+            case 4: DLM_LROWS_H(2, 16); break;
+            case 6: DLM_LROWS_H(6, 8); break;
+            default: DLM_LROWS_H(4, 16); break;
         }
 #undef DLM_LROWS_H
 #undef DLM_LROWS
