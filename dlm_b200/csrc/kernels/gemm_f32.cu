@@ -121,8 +121,9 @@ __device__ __forceinline__ void store4(const F32Params& p, int row, int col, con
 // ------------------------------------------------------------------------------------------------ many rows
 constexpr int TBK = 16;
 
+// (512 threads a multiprocessor, 128 registers each: with the 130 the compiler takes by itself there is room for 256)
 template <int BM, int BN, int EPI>
-__global__ void __launch_bounds__((BM / 8) * (BN / 8)) gemm_f32_tile_kernel(F32Params p) {
+__global__ void __launch_bounds__((BM / 8) * (BN / 8), 512 / ((BM / 8) * (BN / 8))) gemm_f32_tile_kernel(F32Params p) {
     constexpr int TX = BN / 8, THREADS = (BM / 8) * TX;
     constexpr int PA = BM + 4, PB = BN + 4;
     constexpr int LA = BM * (TBK / 4) / THREADS, LB = BN * (TBK / 4) / THREADS;     // 16-byte loads a thread and slice
