@@ -150,11 +150,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    const int r = s_map[0];
-    if (r < 0) {                                           // uniform over the block; nothing allocated yet
-        dep_wait();                                        // (every block waits for the kernel before, see common.cuh)
-        return;
-    }
+    const int r = s_map[0];                                // (the lengths are the step's inputs, not a kernel's output)
+    // every block waits for the kernel before this one (see common.cuh), and takes tensor memory only when it has ended
+    dep_wait();
+    if (r < 0) return;                                     // uniform over the block; nothing allocated yet
     if (warp == MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                      "r"(TMEM_COLS) : "memory");
@@ -165,8 +164,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_slot;
     volatile int* abort_flag = &s_abort;
-    // the set-up above may run while the kernel before this one ends (see dep_wait in common.cuh)
-    dep_wait();
     dep_launch_next();
 
     const int q0 = s_map[1];

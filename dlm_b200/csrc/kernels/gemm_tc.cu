@@ -77,10 +77,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], EPI_WARPS * 32); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = tid; i < TABLE; i += THREADS) {
+    // Nothing an earlier kernel wrote is read, and nothing another block could wait for is taken, before the kernel
+    // before this one has ended: a block made resident early that looked up the offsets then need not see what the
+    // routing wrote.
+    dep_wait();
+    for (int i = warp; i < TABLE; i += THREADS / 32) {
         const long long tile = (long long)blockIdx.x + (long long)i * gridDim.x;
-        if (tile < total_tiles) s_tiles[i] = tile_info(p, (int)(tile / nx));
+        if (tile >= total_tiles) break;
+        const TileInfo ti = tile_info_warp(p, (int)(tile / nx), TT);
+        if (lane == 0) s_tiles[i] = ti;
     }
+    __syncwarp();
     if (warp == MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                      "r"((uint32_t)(2 * TT)) : "memory");
@@ -96,8 +103,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const int i = (tile - (int)blockIdx.x) / (int)gridDim.x;
         return i < TABLE ? s_tiles[i] : tile_info(p, tile / nx);
     };
-    // the set-up above may run while the kernel before this one ends (see dep_wait in common.cuh)
-    dep_wait();
     dep_launch_next();
 
     if (warp == PRODUCER_WARP) {

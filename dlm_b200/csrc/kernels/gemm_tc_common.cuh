@@ -53,6 +53,37 @@ __device__ __forceinline__ TileInfo tile_info(const TcParams& p, int ty, int tt 
     return t;
 }
 
+// The same, asked by a whole warp: the offsets are read 32 experts at a time and every lane gets the answer.
+__device__ __forceinline__ TileInfo tile_info_warp(const TcParams& p, int ty, int tt) {
+    if (p.expert_offsets == nullptr) return tile_info(p, ty, tt);
+    const int lane = threadIdx.x & 31;
+    TileInfo t{-1, 0, 0};
+    int acc = 0;
+    for (int base = 0; base < p.num_experts; base += 32) {
+        const int e = base + lane;
+        const int r0 = e < p.num_experts ? p.expert_offsets[e] : 0, r1 = e < p.num_experts ? p.expert_offsets[e + 1] : 0;
+        const int tiles_e = (r1 - r0 + tt - 1) / tt;
+        int upto = tiles_e;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, ty < acc + upto);
+        if (hit != 0) {
+            const int src = __ffs(hit) - 1;
+            const int before = acc + __shfl_sync(0xffffffffu, upto - tiles_e, src);
+            t.expert = base + src;
+            t.row_begin = __shfl_sync(0xffffffffu, r0, src) + (ty - before) * tt;
+            t.row_end = min(min(__shfl_sync(0xffffffffu, r1, src), t.row_begin + tt), p.M);
+            if (t.row_begin >= t.row_end) t.expert = -1;
+            break;
+        }
+        acc += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return t;
+}
+
 // Token tiles are fetched with the smallest of sixteen boxes that holds the tile's tokens (16, 32, ..., 256
 // rows; half of that where a pair of multiprocessors shares a tile), so that a short group does not cost the
 // bandwidth of a full one.

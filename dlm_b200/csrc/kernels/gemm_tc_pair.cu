@@ -115,10 +115,18 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * EPI_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = tid; i < TABLE; i += THREADS) {
+    // Nothing an earlier kernel wrote is read before the kernel before this one has ended.  A block made resident early
+    // that looked up the offsets then need not see what the routing wrote, and two blocks of a pair that see different
+    // offsets build different tile lists: one waits for an accumulator that the other never delivers.  Nor is tensor
+    // memory taken, or the partner waited for, while that kernel runs.
+    dep_wait();
+    for (int i = warp; i < TABLE; i += THREADS / 32) {
         const long long tile = (long long)pair + (long long)i * n_pairs;
-        if (tile < total_tiles) s_tiles[i] = tile_info(p, (int)(tile / nx), tt);
+        if (tile >= total_tiles) break;
+        const TileInfo ti = tile_info_warp(p, (int)(tile / nx), tt);
+        if (lane == 0) s_tiles[i] = ti;
     }
+    __syncwarp();
     if (warp == MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                      "r"((uint32_t)(2 * TT)) : "memory");
@@ -135,7 +143,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const int i = (tile - pair) / n_pairs;
         return i < TABLE ? s_tiles[i] : tile_info(p, tile / nx, tt);
     };
-    dep_wait();
     dep_launch_next();
 
     if (warp == PRODUCER_WARP) {

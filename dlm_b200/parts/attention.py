@@ -181,11 +181,9 @@ def latent_attend(ops, q, gate, w_ukT, w_uv, sink, cache, block_table, batch, in
     dv = w_uv.shape[1]
     T = q.shape[0]
     dr = q.shape[1] // H - dn
-    # (asked for before the split: the grouped products look their offsets up while the kernel launched just before them
-    # still runs, so the one that writes them must lie further back)
-    offsets = ops.head_offsets(H, T, q.device)
     qn, q_rot = ops.latent_q_split(q, batch.positions, inv_freq, rot_dims, H, dn, dr, cache.dtype,
                                    interleaved=interleaved)
+    offsets = ops.head_offsets(H, T, q.device)
     q_lat = ops.grouped_linear(qn.reshape(H * T, dn), w_ukT, offsets).reshape(H, T, rank)
     lat = ops.latent_attention(q_lat, q_rot, sink, cache, block_table, batch, H, dr, rank, window, scale)
     val = ops.grouped_linear(lat.reshape(H * T, rank), w_uv, offsets)

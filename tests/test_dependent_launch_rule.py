@@ -1,0 +1,42 @@
+"""The rule that kernels launched with programmatic dependent launch keep (``dep_wait`` in common.cuh), read off their
+sources: a race that it excludes shows on a device only now and then."""
+import glob
+import os
+import re
+
+import pytest
+
+SOURCES = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "dlm_b200", "csrc", "kernels")
+
+
+def kernels():
+    """``(file, name, parameters, body)`` of every kernel that waits for the kernel before it; comments taken out."""
+    out = []
+    for path in sorted(glob.glob(os.path.join(SOURCES, "*.cu"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__", text):
+            head_end = text.index(") {\n", m.start())
+            head, body = text[m.start():head_end], text[head_end:text.index("\n}\n", head_end)]
+            if "dep_wait()" in body:
+                head = re.sub(r"__launch_bounds__\((?:[^()]|\((?:[^()]|\([^()]*\))*\))*\)", "", head)
+                name = re.search(r"(\w+)\s*\(", head).group(1)
+                out.append((os.path.basename(path), name, head[head.index(name) + len(name) + 1:], body))
+    return out
+
+
+KERNELS = kernels()
+
+
+def test_the_kernels_were_found():
+    names = {k[1] for k in KERNELS}
+    assert {"gemm_tc_kernel", "gemm_tc_pair_kernel", "gemm_stream_kernel", "attention_prefill_tc_kernel",
+            "rmsnorm_kernel", "causal_conv_runs_kernel"} <= names
+
+
+@pytest.mark.parametrize("file,name,params,body", KERNELS, ids=[f"{k[0]}:{k[1]}" for k in KERNELS])
+def test_nothing_is_looked_up_or_taken_before_the_wait(file, name, params, body):
+    """Offsets of groups are an earlier kernel's output; tensor memory and a cluster's barrier are what another block may
+    wait for."""
+    before = body[:body.index("dep_wait()")]
+    for word in ("tile_info", "expert_offsets[", "tcgen05.alloc", "cluster_sync_all"):
+        assert word not in before, f"{name} uses {word} before it waits for the kernel before it"
