@@ -90,6 +90,12 @@ router_logits_kernel(const TX* h, const T* __restrict__ w, const float* __restri
     if (lane == 0) logits[(long long)t * rows + e] = s;
 }
 
+// A load in front of dep_wait() of what the kernel before the last one, or one before it, wrote.  That kernel has ended
+// and its writes are in L2: the last kernel's blocks all waited for it before they let this one be made resident.  What
+// nobody has waited for on this multiprocessor's behalf is its L1, which may still hold the address as it was; the load
+// goes past it.
+template <typename TX> __device__ __forceinline__ TX load_settled(const TX* p) { return __ldcg(p); }
+
 // The same for many tokens: a block takes ROUTER_TB tokens, so that a weight row read from memory meets all
 // of them.  Per token the sums run in exactly the order of router_logits_kernel, so a token's logits do not
 // depend on which of the two kernels computed them.
@@ -104,6 +110,7 @@ router_logits_multi_kernel(const TX* h, const T* __restrict__ w, const float* __
     extern __shared__ float smem[];               // [ROUTER_TB][H]
     // x_settled: the activations are older than the kernel launched just before this one; the tokens are
     // staged and a warp's first sums worked out while that kernel ends, and nothing is stored before the wait
+    // (see load_settled)
     bool waited = x_settled == 0;
     if (waited) {
         dep_wait();
@@ -131,7 +138,7 @@ router_logits_multi_kernel(const TX* h, const T* __restrict__ w, const float* __
                 for (int v = 0; v < ROUTER_WARPS; ++v) {
                     const int i = base + 32 * v + lane;
                     if (i < H) {
-                        const float val = to_f32(src[i]);
+                        const float val = to_f32(load_settled(src + i));
                         x[i] = val;
                         part[v] = fmaf(val, val, part[v]);
                     }
@@ -351,7 +358,7 @@ router_fused_kernel(const TX* h, const T* __restrict__ w, const float* __restric
         if (e_mine < rows) prefetch_row_l2(w + (long long)e_mine * H, H, threadIdx.x & 31);
     }
     // x_settled: the activations are older than the kernel launched just before this one (the caller says so),
-    // and the logits are worked out while that kernel ends; nothing is written before the wait.
+    // and the logits are worked out while that kernel ends; nothing is written before the wait. (See load_settled.)
     if (!x_settled) {
         dep_wait();
         dep_launch_next();
@@ -360,7 +367,7 @@ router_fused_kernel(const TX* h, const T* __restrict__ w, const float* __restric
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float ss = 0.f;
     for (int i = tid; i < H; i += blockDim.x) {
-        const float v = to_f32(h[(long long)t * H + i]);
+        const float v = to_f32(load_settled(h + (long long)t * H + i));
         x[i] = v;
         ss = fmaf(v, v, ss);
     }

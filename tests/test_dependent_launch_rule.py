@@ -40,3 +40,9 @@ def test_nothing_is_looked_up_or_taken_before_the_wait(file, name, params, body)
     before = body[:body.index("dep_wait()")]
     for word in ("tile_info", "expert_offsets[", "tcgen05.alloc", "cluster_sync_all"):
         assert word not in before, f"{name} uses {word} before it waits for the kernel before it"
+
+
+@pytest.mark.parametrize("name", ["router_logits_multi_kernel", "router_fused_kernel"])
+def test_a_router_that_reads_before_the_wait_reads_past_l1(name):
+    (body,) = [k[3] for k in KERNELS if k[1] == name]
+    assert "load_settled(" in body and not re.search(r"to_f32\((?:src|h)\[", body)
