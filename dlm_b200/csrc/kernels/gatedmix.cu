@@ -313,11 +313,11 @@ __global__ void gated_scan_kernel(const float* __restrict__ q, int ldq, const fl
 // are rotated first and then divided by their root mean square, without weights (the rotated head stays in shared
 // memory until its sum is there).  Without slots only the query heads are read.
 template <typename T, bool AFTER>
-__global__ void head_norm_rope_write_kernel(const float* __restrict__ qkv, int ld, const int32_t* __restrict__ positions,
+__global__ void head_norm_rope_write_kernel(const float* qkv, int ld, const int32_t* __restrict__ positions,
                                             const float* __restrict__ qn_w, const float* __restrict__ kn_w, float eps,
                                             const float* __restrict__ inv_freq, int rot_dims, int interleaved,
-                                            float amplitude, const int32_t* __restrict__ slots, T* __restrict__ q_out,
-                                            T* __restrict__ k_cache, T* __restrict__ v_cache, int nh, int nkv, int d,
+                                            float amplitude, const int32_t* __restrict__ slots, T* q_out,
+                                            T* k_cache, T* v_cache, int nh, int nkv, int d,
                                             int dv, int D, int page_size, int total_pages,
                                             int* err) {
     dep_wait();
@@ -431,9 +431,9 @@ __global__ void head_gate_kernel(T* o, const float* gate, int ldg, int nh, int D
 // `staged`: the two rows are read from global memory once, side by side, and kept in shared memory ([2][H]) for the
 // later passes (a thread rereads only its own entries); otherwise the later passes read global memory again.
 template <typename T>
-__global__ void norm_add_norm_kernel(float* __restrict__ resid, const float* __restrict__ y,
+__global__ void norm_add_norm_kernel(float* resid, const float* y,
                                      const float* __restrict__ w_post, const float* __restrict__ w_next, float eps,
-                                     T* __restrict__ out, int H, int staged) {
+                                     T* out, int H, int staged) {
     dep_wait();
     dep_launch_next();
     __shared__ float s_part[32];

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_smallm_kernel(SmallParams p) 
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt) {
                         uint4 xb = make_uint4(0, 0, 0, 0);
-                        if (in && arow[nt] != nullptr) xb = __ldg(reinterpret_cast<const uint4*>(arow[nt] + k));
+                        if (in && arow[nt] != nullptr) xb = *reinterpret_cast<const uint4*>(arow[nt] + k);
                         mma_bf16(acc[nt], wa[u][0].x, wa[u][1].x, wa[u][0].y, wa[u][1].y, xb.x, xb.y);
                         mma_bf16(acc[nt], wa[u][0].z, wa[u][1].z, wa[u][0].w, wa[u][1].w, xb.z, xb.w);
                     }

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_stream_kernel(StreamParams p)
                 for (int b = 0; b < 8; ++b) {
                     xb[nt][XO + b] = make_uint4(0, 0, 0, 0);
                     if (b < nb && arow != nullptr && kw + 32 * b + 8 * t < len)
-                        xb[nt][XO + b] = __ldg(reinterpret_cast<const uint4*>(arow + 32 * b));
+                        xb[nt][XO + b] = *reinterpret_cast<const uint4*>(arow + 32 * b);
                 }
             }
         };

@@ -25,7 +25,7 @@ namespace {
 // of the token's slot, [rank | dr].  Rotation: entry i < rot_dims / 2 pairs with i + rot_dims / 2, angle
 // position * inv_freq[i] in 32-bit; entries from rot_dims on pass unchanged.
 template <typename T>
-__global__ void latent_prep_kernel(const float* __restrict__ proj, int ld, int off_q, int q_rank,
+__global__ void latent_prep_kernel(const float* proj, int ld, int off_q, int q_rank,
                                    const float* __restrict__ qn_w, int off_kv, int rank, const float* __restrict__ kvn_w,
                                    int dr, const float* __restrict__ inv_freq, int rot_dims, int interleaved,
                                    const int32_t* __restrict__ positions, const int32_t* __restrict__ slots, float eps,
@@ -93,7 +93,7 @@ template <> struct Vec16<__nv_bfloat16> { static constexpr int n = 8; };
 // head by head to qn[H, T, dn] in the activation dtype (the left operand of the per-head product with W_uk), the
 // rotated parts, rotated, to qr[T, H, dr] in 32-bit.
 template <typename T>
-__global__ void latent_q_split_kernel(const float* __restrict__ q, int ldq, const int32_t* __restrict__ positions,
+__global__ void latent_q_split_kernel(const float* q, int ldq, const int32_t* __restrict__ positions,
                                       const float* __restrict__ inv_freq, int rot_dims, int interleaved, T* qn,
                                       float* qr, int Tn, int H, int dn, int dr) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
@@ -133,7 +133,7 @@ __global__ void latent_q_split_kernel(const float* __restrict__ q, int ldq, cons
 // out[t, h * dv + d] = val[h * T + t, d] * sigmoid(gate[t, h])  (gate == nullptr: 1): the per-head values back
 // token by token, gated, in the activation dtype.
 template <typename T>
-__global__ void latent_gate_out_kernel(const float* __restrict__ val, const float* __restrict__ gate, int ldg, T* out,
+__global__ void latent_gate_out_kernel(const float* val, const float* gate, int ldg, T* out,
                                        int Tn, int H, int dv) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
@@ -803,7 +803,7 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
 
 // Merges the splits of a (token, head) in order and normalises as above.  One block a (token, head).
 template <typename T>
-__global__ void latent_merge_kernel(const float* __restrict__ partial, int n_splits, const float* __restrict__ sink,
+__global__ void latent_merge_kernel(const float* partial, int n_splits, const float* __restrict__ sink,
                                     T* lat, int Tn, int H, int rank) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();

@@ -38,7 +38,7 @@ __global__ void add_rows_kernel(float* x, const T* __restrict__ table, const int
 }
 
 // ----------------------------------------------------------------- residual streams
-__global__ void streams_expand_kernel(const float* __restrict__ x, float* xs, int S, int H) {
+__global__ void streams_expand_kernel(const float* x, float* xs, int S, int H) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
     const int t = blockIdx.x;
@@ -54,7 +54,7 @@ __global__ void streams_expand_kernel(const float* __restrict__ x, float* xs, in
 // One block a token; u is kept in shared memory between the two passes.  The sum of squares is added in a fixed
 // order: per-thread partial sums over i = tid, tid + 256, ..., a shuffle tree per warp, the warps in order.
 template <typename TOut>
-__global__ void streams_reduce_kernel(const float* __restrict__ xs, const float* __restrict__ a,
+__global__ void streams_reduce_kernel(const float* xs, const float* __restrict__ a,
                                       const float* __restrict__ norm_w, float eps, TOut* out, int S, int H) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
@@ -85,7 +85,7 @@ __global__ void streams_reduce_kernel(const float* __restrict__ xs, const float*
 constexpr int MAX_STREAMS = 16;
 template <int SC>
 __global__ void streams_update_kernel(float* xs, const float* __restrict__ mix, const float* __restrict__ outw,
-                                      const float* __restrict__ y, int H) {
+                                      const float* y, int H) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
     __shared__ float s_mix[SC * SC], s_out[SC];
@@ -113,7 +113,7 @@ __global__ void streams_update_kernel(float* xs, const float* __restrict__ mix, 
 // out = rmsnorm(sum_r in_next[r] xs_new[t, r, :]) * norm_w (norm_w == nullptr: the sum itself).  One block a token.
 template <int SC, typename TOut>
 __global__ void streams_update_reduce_kernel(float* xs, const float* __restrict__ mix, const float* __restrict__ outw,
-                                             const float* __restrict__ y, const float* __restrict__ in_next,
+                                             const float* y, const float* __restrict__ in_next,
                                              const float* __restrict__ norm_w, float eps, TOut* out, int H) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
@@ -161,8 +161,8 @@ __global__ void streams_update_reduce_kernel(float* xs, const float* __restrict_
 // Inputs before the first token of this step come from the request's carried inputs, state[slot, taps - 1, C]
 // (oldest first; zeros when the request starts).
 template <typename TOut>
-__global__ void causal_conv_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w,
-                                   const float* __restrict__ bias, const float* __restrict__ state,
+__global__ void causal_conv_kernel(const float* x, int ldx, const float* __restrict__ w,
+                                   const float* __restrict__ bias, const float* state,
                                    const int32_t* __restrict__ cu_q, const int32_t* __restrict__ token_req,
                                    const int32_t* __restrict__ state_slot, int C, int taps, int add_input, int act,
                                    TOut* out, int ldo) {
@@ -199,8 +199,8 @@ __device__ __forceinline__ void store4(__nv_bfloat16* o, const float (&v)[4]) {
 // a run.  The sums are those of the kernel above.  Bound by memory; the block a token above read every input and every weight
 // TAPS times, 4 bytes at a time (2,048 tokens x 2,048 channels to bfloat16: 33 -> 15 us, 0.26 of copy bandwidth).
 template <int TAPS, typename TOut>
-__global__ void causal_conv_runs_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w,
-                                        const float* __restrict__ bias, const float* __restrict__ state,
+__global__ void causal_conv_runs_kernel(const float* x, int ldx, const float* __restrict__ w,
+                                        const float* __restrict__ bias, const float* state,
                                         const int32_t* __restrict__ cu_q, const int32_t* __restrict__ token_req,
                                         const int32_t* __restrict__ state_slot, int T, int C, int run, int add_input, int act,
                                         TOut* out, int ldo) {
@@ -265,7 +265,7 @@ __global__ void causal_conv_runs_kernel(const float* __restrict__ x, int ldx, co
 // The carried inputs after the step: the last taps - 1 of (old carried inputs, this step's inputs).  One thread
 // owns a (request, channel): it reads what it needs before it writes.
 constexpr int MAX_TAPS = 16;
-__global__ void conv_state_kernel(const float* __restrict__ x, int ldx, float* state, const int32_t* __restrict__ cu_q,
+__global__ void conv_state_kernel(const float* x, int ldx, float* state, const int32_t* __restrict__ cu_q,
                                   const int32_t* __restrict__ state_slot, int C, int taps, int skip_single) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
@@ -286,7 +286,7 @@ __global__ void conv_state_kernel(const float* __restrict__ x, int ldx, float* s
 
 // -------------------------------------------------------------------- activations
 template <typename TOut>
-__global__ void activation_kernel(const float* __restrict__ x, int ldx, TOut* out, int ldo, int cols, int op) {
+__global__ void activation_kernel(const float* x, int ldx, TOut* out, int ldo, int cols, int op) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
     const int r = blockIdx.x;
@@ -331,7 +331,7 @@ __global__ void table_lookup_kernel(const int32_t* __restrict__ tokens, const in
 // One block a (token, group) of `gs` channels.  mode 0: v = y * silu(gate); out = v / rms(v) * w.
 // mode 1: out = y / rms(y) * w * sigmoid(gate).  rms over the group, eps inside the root.
 template <typename TOut>
-__global__ void gated_rmsnorm_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ gate, int ldg,
+__global__ void gated_rmsnorm_kernel(const float* y, int ldy, const float* gate, int ldg,
                                      const float* __restrict__ w, TOut* out, int ldo, int gs, float eps, int mode,
                                      const float* row_scale) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended

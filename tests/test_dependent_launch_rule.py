@@ -46,3 +46,20 @@ def test_nothing_is_looked_up_or_taken_before_the_wait(file, name, params, body)
 def test_a_router_that_reads_before_the_wait_reads_past_l1(name):
     (body,) = [k[3] for k in KERNELS if k[1] == name]
     assert "load_settled(" in body and not re.search(r"to_f32\((?:src|h)\[", body)
+
+
+# weights, tables and constants, and what the host copies to the device before a step's first kernel
+NO_KERNEL_WRITES = set("""w b w2 b2 wa wb w_post w_next norm_w qn_w kn_w kvn_w bias vec sink sinks slopes select_bias table added a mix
+    outw in_next inv_freq tokens idx positions slots block_table cu_q kv_len token_req state_slot""".split())
+
+
+@pytest.mark.parametrize("file,name,params,body", KERNELS, ids=[f"{k[0]}:{k[1]}" for k in KERNELS])
+def test_what_kernels_write_is_not_declared_read_only(file, name, params, body):
+    """A load through a ``__restrict__`` pointer to const may take the path for data that nothing writes while the kernel is
+    resident, or move above the wait; so may ``__ldg``."""
+    text = open(os.path.join(SOURCES, file)).read()
+    launched_early = re.search(r"launch_dep\(\s*" + name + r"\b", text) or (
+        re.search(r"launch_dep\(\s*kern\b", text) and re.search(r"kern = [^;]*\b" + name + r"\b", text))
+    if launched_early:
+        assert set(re.findall(r"__restrict__ (\w+)", params)) <= NO_KERNEL_WRITES
+        assert set(re.findall(r"__ldg\([^;]*?(\w+) \+", body)) <= {"w4"}
