@@ -140,7 +140,7 @@ int take_error_flag();
 void reset_decode_merge_counters(cudaStream_t stream);
 
 // Whether the small kernels are launched so that each may start while the one before it ends
-// (programmatic dependent launch; on unless DLM_B200_NO_PDL=1).
+// (programmatic dependent launch; on unless DLM_B200_NO_PDL=1).  Setting it concerns the calling thread only.
 bool dep_launch_enabled();
 void set_dep_launch(bool on);
 

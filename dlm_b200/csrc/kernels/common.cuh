@@ -70,7 +70,8 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 __device__ __forceinline__ void dep_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Whether launch_dep() asks for the early launch (off: DLM_B200_NO_PDL=1, or set_dep_launch(false)).
+// Whether launch_dep() asks for the early launch (off: DLM_B200_NO_PDL=1, or set_dep_launch(false), which holds for the
+// calling thread's launches only).
 bool dep_launch_enabled();
 void set_dep_launch(bool on);
 

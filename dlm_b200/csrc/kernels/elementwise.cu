@@ -26,17 +26,17 @@ int* error_flag_ptr() {
 }
 
 namespace {
-int g_dep_launch = -1;
+thread_local int t_dep_launch = -1;       // -1: this thread has not set it
 }
 
 bool dep_launch_enabled() {
-    if (g_dep_launch < 0) {
+    static const bool wanted = [] {
         const char* off = std::getenv("DLM_B200_NO_PDL");
-        g_dep_launch = (off != nullptr && off[0] != '\0' && off[0] != '0') ? 0 : 1;
-    }
-    return g_dep_launch == 1;
+        return !(off != nullptr && off[0] != '\0' && off[0] != '0');
+    }();
+    return t_dep_launch < 0 ? wanted : t_dep_launch == 1;
 }
-void set_dep_launch(bool on) { g_dep_launch = on ? 1 : 0; }
+void set_dep_launch(bool on) { t_dep_launch = on ? 1 : 0; }
 
 int sm_count() {
     static int n = 0;

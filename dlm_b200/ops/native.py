@@ -93,14 +93,14 @@ class NativeOps:
         return _Branch(self._side)
 
     def dependent_launch(self, on: bool):
-        """A context in which the short kernels are (on) or are not (off) launched with programmatic dependent
-        launch; the library's setting is put back at the end."""
+        """A context in which the short kernels that this thread launches are (on) or are not (off) launched with
+        programmatic dependent launch; the thread's setting is put back at the end."""
         import contextlib
 
         @contextlib.contextmanager
         def scope():
             before = bool(self.k.dep_launch_enabled())
-            self.k.set_dep_launch(bool(on) and before)      # never switched on where the process has it off
+            self.k.set_dep_launch(bool(on) and before)      # never switched on where it is off
             try:
                 yield
             finally:

@@ -3,6 +3,7 @@ sources: a race that it excludes shows on a device only now and then."""
 import glob
 import os
 import re
+import threading
 
 import pytest
 
@@ -63,3 +64,38 @@ def test_what_kernels_write_is_not_declared_read_only(file, name, params, body):
     if launched_early:
         assert set(re.findall(r"__restrict__ (\w+)", params)) <= NO_KERNEL_WRITES
         assert set(re.findall(r"__ldg\([^;]*?(\w+) \+", body)) <= {"w4"}
+
+
+def test_the_setting_belongs_to_a_thread():
+    """Two engines in two threads, one of a design that asks for ordinary launches: neither changes the other's setting, and
+    both find their own as it was whichever ends first."""
+    from dlm_b200.build import load_kernels
+    from dlm_b200.ops.native import NativeOps
+    ops = NativeOps.__new__(NativeOps)
+    ops.k = load_kernels()
+    before = bool(ops.k.dep_launch_enabled())
+    entered, leave, seen = threading.Event(), threading.Event(), []
+
+    def other():
+        ops.k.set_dep_launch(True)
+        with ops.dependent_launch(False):
+            entered.set()
+            assert leave.wait(30)
+            seen.append(bool(ops.k.dep_launch_enabled()))
+        seen.append(bool(ops.k.dep_launch_enabled()))
+
+    t = threading.Thread(target=other)
+    try:
+        ops.k.set_dep_launch(True)
+        t.start()
+        assert entered.wait(30)
+        seen.append(bool(ops.k.dep_launch_enabled()))      # this thread's, while the other has it off
+        with ops.dependent_launch(False):
+            leave.set()
+            t.join()
+            seen.append(bool(ops.k.dep_launch_enabled()))  # the other has put its own back
+        seen.append(bool(ops.k.dep_launch_enabled()))
+    finally:
+        leave.set()
+        ops.k.set_dep_launch(before)
+    assert seen == [True, False, True, False, True]
