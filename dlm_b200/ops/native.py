@@ -576,15 +576,32 @@ class NativeOps:
                            dk, dv, float(q_scale), float(den_eps), self._stream())
         return o, rden
 
+    most_head_offsets = 4096      # tensors of head_offsets kept for steps that are not replayed
+
+    @staticmethod
+    def _capturing(device) -> bool:
+        return torch.device(device).type == "cuda" and torch.cuda.is_current_stream_capturing()
+
     def head_offsets(self, H, T, device):
-        """``[0, T, 2T, ..., H T]``: the groups of a grouped product whose groups are heads (kept: built once)."""
+        """``[0, T, 2T, ..., H T]``: the groups of a grouped product whose groups are heads (kept: built once).
+        A recorded graph holds the tensor's address, so one that a recording has asked for is never given up; one
+        that is first asked for during a recording belongs to the graph, which fills it at every replay."""
         key = (H, T, str(device))
         cache = self.__dict__.setdefault("_head_offsets", {})
-        if key not in cache:
-            if len(cache) > 4096:
-                cache.clear()
-            cache[key] = torch.arange(0, (H + 1) * T, T, dtype=torch.int32, device=device)
-        return cache[key]
+        in_graphs = self.__dict__.setdefault("_graph_head_offsets", {})
+        off = in_graphs.get(key)
+        if off is None:
+            off = cache.get(key)
+            recording = self._capturing(device)
+            if off is None:
+                off = torch.arange(0, (H + 1) * T, T, dtype=torch.int32, device=device)
+                if not recording:
+                    if len(cache) >= self.most_head_offsets:
+                        cache.clear()
+                    cache[key] = off
+            elif recording:
+                in_graphs[key] = off
+        return off
 
     def latent_attention(self, q_lat, q_rot, sink, cache, block_table, batch, H, dr, rank, window, scale):
         """Windowed attention over the cached latents with a sink per head.  ``q_lat [H, T, rank]`` (32-bit): the
