@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(32 * MOST_WARPS, 1) scan_walk_kernel(WalkParam
     const float dcoef = MODE == WALK_HEAD && p.D != nullptr ? p.D[h] : 0.f;
     float* st = p.state + ((long long)p.state_slot[r] * p.heads + h) * (long long)N * P;
     auto row_of = [&](int i) { return 4 * rlane + (i & 3) + 4 * RL * (i >> 2); };     // i = 0 .. 7
-    const bool vec = P % CPL == 0;
+    const bool vec = p.state_vec != 0;
     f2 s[4][CPL];                                          // rows (2 i, 2 i + 1) of the lane's columns
     {
         float raw[8][CPL];
@@ -444,6 +444,7 @@ void launch_walk(WalkParams p, int R, int walkers, cudaStream_t stream) {
     const int cols = walkers * CW;
     const int row = walk_vectors<MODE>() * 8 * RL + ((cols + 3) & ~3) + 4;
     p.walkers = walkers;
+    p.state_vec = p.P % CPL == 0 && reinterpret_cast<uintptr_t>(p.state) % (CPL * sizeof(float)) == 0 ? 1 : 0;
     p.wide_v = p.wide && cols % 4 == 0 ? 1 : 0;              // (a block's first column is a multiple of `cols`)
     p.tile = 16;
     while (p.tile > 1 && (size_t)STAGES * p.tile * row * sizeof(float) > 150 * 1024) p.tile /= 2;

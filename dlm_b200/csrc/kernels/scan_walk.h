@@ -25,8 +25,8 @@ struct WalkParams {
     int heads, q_div, N, P;
     int silu_inputs, unit;
     float unit_eps, q_scale, inv_tau, decay_coef;
-    int wide, wide_v, walkers, tile;     // filled in by scan_walk: 16-byte copies are possible (of the vectors, of v); warps
-                                         // that walk; tokens a tile
+    int wide, wide_v, state_vec, walkers, tile;      // filled in by scan_walk: 16-byte copies are possible (of the vectors, of
+                                         // v), a lane's columns of the state come as one access; warps that walk; tokens a tile
 };
 
 // False when the sizes are not its: the caller takes the kernel it has for any size.

@@ -1,0 +1,57 @@
+"""The scans on states at any address, and on steps of few tokens: a request cut into steps of one to four tokens gives the
+bits of the request in one step, whatever kernel the step's lengths choose."""
+import pytest
+import torch
+
+from test_zesapel_gpu import batch_of, randn
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+SIZES = [(1, 1), (8, 2), (9, 3), (16, 4), (17, 7), (32, 66), (33, 5), (64, 64), (65, 12), (128, 33), (129, 8), (256, 6)]
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from dlm_b200.ops import native_ops
+    return native_ops(fast=True)
+
+
+def scans(ops, N, P, T, heads=3):
+    """The four walks (and retention) as functions of (first token, end, batch, state)."""
+    xbc, dt = randn(T, heads * P + 2 * N, seed=1), randn(T, heads, seed=2)
+    bias, A_log, D = randn(heads, seed=3, std=0.5), randn(heads, seed=4, std=0.5), randn(heads, seed=5)
+    q, k, v, z = (randn(T, heads * n, seed=7 + i) for i, n in enumerate((N, N, P, N)))
+    dec, beta, fixed = randn(T, heads, seed=11), randn(T, heads, seed=12), torch.linspace(0.8, 0.99, heads, device=DEV)
+    vkq = torch.cat([v, k, q], 1)
+    proj, lw, a_bias = randn(T, 4 * heads * N, seed=14), randn(T, heads * N, seed=15), randn(heads * N, seed=16)
+    scale = N ** -0.5
+    out = {
+        "ssm": lambda a, e, b, s: ops.ssm_scan(xbc[a:e], dt[a:e], bias, A_log, D, s, b, heads, P, N, 1),
+        "ssm, silu": lambda a, e, b, s: ops.ssm_scan(xbc[a:e].clone(), dt[a:e], bias, A_log, D, s, b, heads, P, N, 1,
+                                                     silu_inputs=True),
+        "retention": lambda a, e, b, s: ops.ssm_scan(vkq[a:e], None, None, None, None, s, b, heads, P, N, heads,
+                                                     fixed_decay=fixed),
+        "channel": lambda a, e, b, s: ops.gated_scan(q[a:e], k[a:e], v[a:e], z[a:e], None, s, b, heads, heads, N, P,
+                                                     q_scale=scale, tau=8.0),
+        "delta": lambda a, e, b, s: ops.gated_scan(q[a:e], k[a:e], v[a:e], dec[a:e], beta[a:e], s, b, heads, heads, N, P,
+                                                   unit_eps=1e-6, q_scale=scale, A_log=A_log, decay_bias=bias),
+    }
+    if N == P:
+        HN = heads * N
+        out["removal"] = lambda a, e, b, s: ops.delta_scan(proj[a:e], (0, HN, 2 * HN, 3 * HN), lw[a:e], a_bias, s, b, heads, N,
+                                                           1e-6, 0.6)
+    return out
+
+
+@pytest.mark.parametrize("N,P", [(16, 4), (64, 64), (128, 36), (24, 6)])
+def test_a_state_may_lie_at_any_address(ops, N, P):
+    """States at storage offsets that are no multiple of 16 bytes (shifted by one number) give what an aligned one gives."""
+    heads, lens = 3, [21, 1, 6]
+    b = batch_of(lens, [2, 0, 3])
+    for name, run in scans(ops, N, P, sum(lens), heads).items():
+        state = randn(5, heads, N, P, seed=6, std=0.3)
+        shifted = torch.empty(state.numel() + 1, device=DEV)[1:].view(state.shape)
+        shifted.copy_(state)
+        want, got = run(0, sum(lens), b, state), run(0, sum(lens), b, shifted)
+        assert torch.equal(got, want) and torch.equal(shifted, state), name
+    ops.check_errors()
