@@ -9,8 +9,7 @@
 namespace dlmk {
 namespace tc5 {
 
-constexpr uint32_t WAIT_LIMIT = 1u << 22;       // try_wait calls before a wait gives up
-constexpr uint64_t WAIT_LIMIT_NS = 2000000000;  // nanoseconds before a wait gives up
+constexpr uint64_t WAIT_LIMIT_NS = 2000000000;  // nanoseconds before a wait on an mbarrier gives up
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -36,20 +35,25 @@ __device__ __forceinline__ uint64_t global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// Bounded wait.  Returns false when it gave up (or another role already had): the caller stops.  The bound is in time
-// (a try may itself block for a while, so a bound in tries alone could last minutes); the clock is read once every 16 tries,
-// which a wait that is met in time hardly ever reaches.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    uint64_t give_up = 0;
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
+// Waits for the phase until the time `give_up` (0: not set yet; the first wait that needs it sets it, so that several waits
+// can share one), or until `abort_flag` (unless that is null) is set.  The bound is in time: a try may itself block for a
+// while, so a bound in tries could last minutes.  The clock is read once every 16 tries, which a wait that is met in time
+// hardly ever reaches.
+__device__ __forceinline__ bool mbar_wait_until(uint64_t* bar, uint32_t parity, uint64_t& give_up, volatile int* abort_flag) {
+    for (uint32_t i = 0;; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
+        if (abort_flag != nullptr && *abort_flag) return false;
         if ((i & 15) == 15) {
             const uint64_t now = global_ns();
             if (give_up == 0) give_up = now + WAIT_LIMIT_NS;
-            else if (now > give_up) break;
+            else if (now > give_up) return false;
         }
     }
+}
+// Bounded wait of a role.  Returns false when it gave up (or another role already had): the caller stops.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    uint64_t give_up = 0;
+    if (mbar_wait_until(bar, parity, give_up, abort_flag)) return true;
     *abort_flag = 1;
     return false;
 }

@@ -66,6 +66,16 @@ def test_what_kernels_write_is_not_declared_read_only(file, name, params, body):
         assert set(re.findall(r"__ldg\([^;]*?(\w+) \+", body)) <= {"w4"}
 
 
+def test_every_wait_on_a_barrier_is_bounded_in_time():
+    """A loop of tries of its own is bounded in tries at best, and each try may block for a while; and a bound in time must not
+    run while the kernel before this one does."""
+    for path in glob.glob(os.path.join(SOURCES, "*.cu")):
+        assert not re.search(r"(?:for|while) \([^\n]*\)[^;{]*\{?\s*(?:if \()?!?mbar_try_wait", open(path).read()), path
+    (body,) = [k[3] for k in KERNELS if k[1] == "gemm_stream_kernel"]
+    producer = body[body.index("if (warp == CW)"):]
+    assert "dep_wait()" in producer[:producer.index("mbar_wait(&empty_bar")]
+
+
 def test_the_setting_belongs_to_a_thread():
     """Two engines in two threads, one of a design that asks for ordinary launches: neither changes the other's setting, and
     both find their own as it was whichever ends first."""
