@@ -7,7 +7,7 @@
 //                   pipe: 32 packed multiply-adds (fma.rn.f32x2, two rounded sums each) meet four 16-byte shared loads.
 //   gemm_f32_few    few rows (a decode step, experts with a few rows each): bound by reading W once.  16 columns a block,
 //                   so that even a product of 2,048 columns spreads over 128 multiprocessors, and a ring of asynchronous copies
-//                   that keeps some 40-90 KB a multiprocessor in flight; a thread owns one column and RPT rows, and the only
+//                   that keeps 32-48 KB a block in flight, 72-86 KB where there are at most two blocks a multiprocessor; a thread owns one column and RPT rows, and the only
 //                   serial chain is the sum itself (4 clocks a k).
 #include "api.h"
 #include "common.cuh"
@@ -339,11 +339,28 @@ void launch_few(const F32Params& p, int m_tiles, cudaStream_t stream) {
     else launch_few_ring<EPI, RPT, false>(p, grid, stream);
 }
 
+// Which kernel: measured at K = 2,048 (all three grow with K alike), beside gemm_simt's 64 x 64 tiles.
+//   few    up to 32 rows (2,048 / 11,264 / 32,768 columns, 32 rows: 29 / 105 / 249 us, gemm_simt 123 / 214 / 364) and up to 16
+//          rows an expert on average (60 experts x 2,816 columns, 8 rows each: 647 us against 1,515; at 12 rows 1,072 against
+//          some 900 of the tiles).  From 33 to 64 rows the weights are read twice: up to 640,000 outputs (64 rows of 6,144 columns:
+//          111 us against 183 of the tiles; 64 rows of 32,768 columns: 488 us, where gemm_simt takes 391).
+//   tile   where gemm_simt would have more than one tile a multiprocessor: its second wave starts there (512 x 2,048: 218 us
+//          against 184; 65 x 6,144: 205 against 183; 2,048 x 2,048: 683 against 433).
+//   none   fewer tiles than that: a thread's 64 sums are then too long a walk (65-256 rows of 2,048 columns: 183 us against 132
+//          of gemm_simt; 128 x 256, K = 256: 27 against 19).
+enum class Plan { none, few, tile };
+Plan plan(int M, int N, int num_experts) {
+    const int mean = num_experts > 0 ? (M + num_experts - 1) / num_experts : M;
+    if (num_experts > 0 ? mean <= 16 : mean <= 32 || (mean <= 64 && (long long)M * N < 640000)) return Plan::few;
+    const long long row_tiles = num_experts > 0 ? (long long)num_experts * (mean / 64 + 1) : (M + 63) / 64;
+    return row_tiles * ((N + 63) / 64) > sm_count() ? Plan::tile : Plan::none;
+}
+
 template <int EPI>
 void launch(const F32Params& p, cudaStream_t stream) {
     const bool grouped = p.expert_offsets != nullptr;
     const int mean = grouped ? (p.M + p.num_experts - 1) / p.num_experts : p.M;
-    if (grouped ? mean <= 16 : mean <= 64) {
+    if (plan(p.M, p.N, grouped ? p.num_experts : 0) == Plan::few) {
         // an expert's rows vary about their mean: the tile holds twice the mean where it can
         const int want = grouped ? 2 * mean : mean;
         const int r = want <= 8 ? 8 : (want <= 16 ? 16 : 32);
@@ -360,8 +377,8 @@ void launch(const F32Params& p, cudaStream_t stream) {
 
 }  // namespace
 
-bool gemm_f32_ok(const void* a, int lda, const void* w, int ldw, long long w_expert_stride, int K) {
-    return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && w_expert_stride % 4 == 0 &&
+bool gemm_f32_takes(const void* a, int lda, const void* w, int ldw, long long w_expert_stride, int M, int N, int K, int num_experts) {
+    return plan(M, N, num_experts) != Plan::none && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && w_expert_stride % 4 == 0 &&
            ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
 }
 

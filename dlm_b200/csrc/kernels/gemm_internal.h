@@ -11,8 +11,9 @@ void gemm_simt(const void* a, int lda, const int32_t* a_rows, const void* w, int
                const int32_t* expert_offsets, int num_experts, const float* bias, void* out, int ldo, int M, int N,
                int K, int in_dtype, int out_dtype, int epilogue, cudaStream_t stream);
 
-// The same sums (bit for bit) for 32-bit inputs and outputs whose rows can be fetched 16 bytes at a time.
-bool gemm_f32_ok(const void* a, int lda, const void* w, int ldw, long long w_expert_stride, int K);
+// The same sums (bit for bit) for 32-bit inputs and outputs whose rows can be fetched 16 bytes at a time, at the sizes where
+// that is faster (num_experts 0: not grouped).
+bool gemm_f32_takes(const void* a, int lda, const void* w, int ldw, long long w_expert_stride, int M, int N, int K, int num_experts);
 void gemm_f32(const float* a, int lda, const int32_t* a_rows, const float* w, int ldw, long long w_expert_stride,
               const int32_t* expert_offsets, int num_experts, const float* bias, float* out, int ldo, int M, int N, int K,
               int epilogue, cudaStream_t stream);

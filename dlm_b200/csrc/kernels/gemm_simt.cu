@@ -161,7 +161,7 @@ void gemm_simt(const void* a, int lda, const int32_t* a_rows, const void* w, int
         m_tiles += num_experts;   // every group may end in a partial tile
     }
     DLM_CHECK(m_tiles <= 65535, "gemm: too many row tiles for one launch");
-    if (in_dtype == F32 && out_dtype == F32 && gemm_f32_ok(a, lda, w, ldw, w_expert_stride, K)) {
+    if (in_dtype == F32 && out_dtype == F32 && gemm_f32_takes(a, lda, w, ldw, w_expert_stride, M, N, K, expert_offsets != nullptr ? num_experts : 0)) {
         gemm_f32(static_cast<const float*>(a), lda, a_rows, static_cast<const float*>(w), ldw, w_expert_stride, expert_offsets,
                  num_experts, bias, static_cast<float*>(out), ldo, M, N, K, epilogue, stream);
         return;
