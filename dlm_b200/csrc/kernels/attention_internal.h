@@ -86,8 +86,8 @@ void attention_simt(const void* q, const void* k_cache, const void* v_cache, con
                     int nkv, int hd, int page_size, int total_pages, int window, Score scale, int skip_single,
                     int dtype, cudaStream_t stream);
 
-// The same results, bit for bit, in 32-bit for the sizes attention_f32_ok names.
-bool attention_f32_ok(const void* q, const void* k_cache, const void* v_cache, int hd, Score scale);
+// The same results, bit for bit, in 32-bit for what attention_f32_takes names.
+bool attention_f32_takes(const void* q, const void* k_cache, const void* v_cache, int T, int R, int hd, Score scale);
 void attention_f32(const float* q, const float* k_cache, const float* v_cache, const int32_t* block_table, int table_width,
                    const int32_t* cu_q, const int32_t* kv_len, float* out, int T, int R, int nh, int nkv, int hd,
                    int page_size, int total_pages, int window, Score scale, int skip_single, cudaStream_t stream);

@@ -1,5 +1,5 @@
-// Paged causal attention on the FMA units, for any head size up to 256 and both dtypes.
-// It is the 32-bit path's attention and the reference every faster kernel is checked against.
+// Paged causal attention on the FMA units, for any head size up to 256 and both dtypes: what the kernels for certain sizes and
+// alignments do not take.  attention_f32.cu gives the same bits in 32-bit.
 //
 // One block = 16 consecutive query tokens of one request x one query head.  Keys are walked
 // in tiles of 32 that start at absolute positions divisible by 32, and a tile in which a
@@ -179,7 +179,7 @@ void attention_simt(const void* q, const void* k_cache, const void* v_cache, con
     if (T <= 0 || R <= 0) return;
     DLM_CHECK(hd > 0 && hd <= MAX_HD, "attention: head_dim must be in 1..256");
     DLM_CHECK(nh % nkv == 0, "attention: heads must be a multiple of kv heads");
-    if (dtype == F32 && attention_f32_ok(q, k_cache, v_cache, hd, scale)) {
+    if (dtype == F32 && attention_f32_takes(q, k_cache, v_cache, T, R, hd, scale)) {
         attention_f32(static_cast<const float*>(q), static_cast<const float*>(k_cache), static_cast<const float*>(v_cache),
                       block_table, table_width, cu_q, kv_len, static_cast<float*>(out), T, R, nh, nkv, hd, page_size,
                       total_pages, window, scale, skip_single, stream);
