@@ -238,8 +238,9 @@ __global__ void causal_conv_runs_kernel(const float* x, int ldx, const float* __
             const int t = t0 + u;
             if (t >= last) break;
             if (t >= end) {
-                do { ++r; end = cu_q[r + 1]; } while (t >= end);
+                r = token_req[t];
                 start = cu_q[r];
+                end = cu_q[r + 1];
                 carried(t);
             }
 #pragma unroll
@@ -920,9 +921,12 @@ void causal_conv(const float* x, int ldx, const float* w, const float* bias, flo
                  int act, void* out, int ldo, int out_dtype, cudaStream_t stream) {
     if (T <= 0 || R <= 0) return;
     DLM_CHECK(taps >= 1 && taps <= MAX_TAPS, "causal_conv: 1 to 16 taps");
-    // From 65 tokens on (a decode step is bound by its launch), four taps, channels in fours: runs of tokens, as long as leaves
-    // eight blocks a multiprocessor.
-    if (T > 64 && taps == 4 && C % 4 == 0 && ldx % 4 == 0 && ldo % 4 == 0 &&
+    // Four taps (what the designs have; other counts keep the kernel above), channels in fours, and enough work: a run is a chain
+    // of loads, which costs some 2 us where the block a token takes no time of its own (512 tokens of 96 channels: 10.0 us against
+    // 8.4 with the kernel that shifts the carried inputs, 512 x 512: 10.4 against 10.5, 512 x 2,048: 12.5 against 16.6, 2,048 x
+    // 6,144: 35 against 105).  Requests of a token or so reload their carried inputs at every token of a run: twice the
+    // work (96 such requests of 2,048 channels: 13.4 against 10.6, 128 of 4,352: 16.6 against 16.6).
+    if (T > 64 && (long long)T * C >= (T >= 2 * R ? 300000 : 500000) && taps == 4 && C % 4 == 0 && ldx % 4 == 0 && ldo % 4 == 0 &&
         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
         const int gy = (C / 4 + 127) / 128;
         int run = 16;
