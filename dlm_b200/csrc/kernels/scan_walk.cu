@@ -229,12 +229,13 @@ __global__ void __launch_bounds__(32 * MOST_WARPS, 1) scan_walk_kernel(WalkParam
                             }
                         }
                     } else {
-                        // k stays as it is (it carries v); the removal's r u u^T S = (r k / |k|^2)(k^T S); q meets the old
-                        // state through the decays
+                        // k stays as it is (it carries v); the removal's r u u^T S = (r k / |k| / |k|)(k^T S): divided twice, so
+                        // that nothing leaves the 32-bit range that u and r u do not leave; q meets the old state through
+                        // the decays
                         qr = token_sum(qr);
-                        const float inv2 = 1.0f / (kk + p.unit_eps);
+                        const float inv = 1.0f / sqrtf(kk + p.unit_eps);
                         if (mine) {
-                            if (lt == 0) row[off_s + 1] = qr * inv2;
+                            if (lt == 0) row[off_s + 1] = qr * inv * inv;
                             if (lt == 1) row[off_s + 2] = qk;
 #pragma unroll
                             for (int q = 0; q < QL; ++q) {
@@ -242,8 +243,8 @@ __global__ void __launch_bounds__(32 * MOST_WARPS, 1) scan_walk_kernel(WalkParam
                                 *reinterpret_cast<float4*>(row + i) = make_float4(qv[4 * q] * av[4 * q], qv[4 * q + 1] * av[4 * q + 1],
                                                                                   qv[4 * q + 2] * av[4 * q + 2], qv[4 * q + 3] * av[4 * q + 3]);
                                 *reinterpret_cast<float4*>(row + 2 * NP + i) = make_float4(av[4 * q], av[4 * q + 1], av[4 * q + 2], av[4 * q + 3]);
-                                *reinterpret_cast<float4*>(row + 3 * NP + i) = make_float4(-rv[4 * q] * inv2, -rv[4 * q + 1] * inv2,
-                                                                                           -rv[4 * q + 2] * inv2, -rv[4 * q + 3] * inv2);
+                                *reinterpret_cast<float4*>(row + 3 * NP + i) = make_float4(-rv[4 * q] * inv * inv, -rv[4 * q + 1] * inv * inv,
+                                                                                           -rv[4 * q + 2] * inv * inv, -rv[4 * q + 3] * inv * inv);
                             }
                         }
                     }

@@ -55,3 +55,25 @@ def test_a_state_may_lie_at_any_address(ops, N, P):
         want, got = run(0, sum(lens), b, state), run(0, sum(lens), b, shifted)
         assert torch.equal(got, want) and torch.equal(shifted, state), name
     ops.check_errors()
+
+
+def test_removal_with_short_keys_and_no_floor(ops):
+    """Keys of length 1e-20: their square is no normal number and its reciprocal out of range, their unit vector is fine."""
+    heads, d, lens = 2, 16, [7, 1]
+    T, b = 8, batch_of([7, 1], [0, 1])
+    proj, lw, a_bias = randn(T, 4 * heads * d, seed=1), randn(T, heads * d, seed=2), randn(heads * d, seed=3)
+    HD = heads * d
+    k = proj[:, HD:2 * HD]
+    small = proj.clone()
+    small[:, HD:2 * HD] = k * 2.0 ** -62       # |k|^2 about 2^-120
+    small[:, 2 * HD:3 * HD] = proj[:, 2 * HD:3 * HD] * 2.0 ** 62
+    tiny = proj.clone()
+    tiny[:, HD:2 * HD] = k * 2.0 ** -67        # |k|^2 about 2^-130, its reciprocal beyond the largest number
+    tiny[:, 2 * HD:3 * HD] = proj[:, 2 * HD:3 * HD] * 2.0 ** 67
+    outs = []
+    for p in (proj, small, tiny):
+        s = randn(2, heads, d, d, seed=4, std=0.3)
+        outs.append((ops.delta_scan(p, (0, HD, 2 * HD, 3 * HD), lw, a_bias, s, b, heads, d, 0.0, 0.6), s))
+    for o, s in outs[1:]:
+        # k v^T is as before and so is the unit vector, up to the bits that |k|^2 = 2^-130 keeps (about 19 of 24)
+        assert torch.allclose(o, outs[0][0], atol=1e-3, rtol=1e-3) and torch.allclose(s, outs[0][1], atol=1e-3, rtol=1e-3)
