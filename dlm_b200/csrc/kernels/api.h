@@ -199,9 +199,11 @@ void gated_rmsnorm(const float* y, int ldy, const float* gate, int ldg, const fl
 // fixed_decay f32 [heads] != nullptr: S <- fixed_decay[head] S + B x^T instead (step size 1; dt_raw, dt_bias and
 // A_log are not read); D == nullptr: no direct term.  silu_inputs != 0: x, B and C pass silu first.  With groups == heads and rows [v | k | q] this is linear
 // attention with a constant decay per head: S <- decay S + k v^T, y = S^T q.
+// (longest, here and in the scans below: tokens of the step's longest request, or a bound of it; 0: not known.  Steps of a few
+// tokens a request take a kernel without the ring of tiles; the results are the same bits.)
 void ssm_scan(const float* xbc, int ldx, const float* dt_raw, int lddt, const float* dt_bias, const float* A_log,
               const float* D, float* state, const int32_t* cu_q, const int32_t* state_slot, float* y, int R, int heads,
-              int P, int N, int groups, const float* fixed_decay, int silu_inputs, cudaStream_t stream);
+              int P, int N, int groups, const float* fixed_decay, int silu_inputs, int longest, cudaStream_t stream);
 
 // Delta-rule scan.  proj f32 rows hold r, k, v and the raw removal rate at the given column offsets (heads * d
 // each); lw f32 [T, heads * d] the raw decay; state f32 [slots, heads, d, d] (key channel, value channel).
@@ -209,7 +211,7 @@ void ssm_scan(const float* xbc, int ldx, const float* dt_raw, int lddt, const fl
 // S <- diag(w) S - (a u)(u^T S) + k v^T; o = S^T r  (o f32 [T, heads * d]).
 void delta_scan(const float* proj, int ld, int off_r, int off_k, int off_v, int off_a, const float* lw, int ldlw,
                 const float* a_bias, float* state, const int32_t* cu_q, const int32_t* state_slot, float* o, int R,
-                int heads, int d, float unit_eps, float decay_coef, cudaStream_t stream);
+                int heads, int d, float unit_eps, float decay_coef, int longest, cudaStream_t stream);
 
 // ---- diagonal state-space scan and mixers that run side by side (scanmix.cu) ----
 
@@ -221,7 +223,7 @@ void delta_scan(const float* proj, int ld, int off_r, int off_k, int off_v, int 
 void selective_scan(const float* x, int ldx, const float* dt_raw, int lddt, const float* bc, int ldbc, const float* z,
                     int ldz, const float* dt_bias, const float* A_log, const float* D, float* state,
                     const int32_t* cu_q, const int32_t* state_slot, void* out, int ldo, int R, int inner, int N,
-                    int out_dtype, cudaStream_t stream);
+                    int out_dtype, int longest, cudaStream_t stream);
 
 // qkv f32 rows [q: nh * d | k: nkv * d | v: nkv * dv] (row stride ld).  q <- q / rms(q over all nh * d entries) * qn_w
 // * (1 + temp_coef * ln(floor((position + 1) / temp_every) + 1)); k likewise with kn_w and no temperature (a weight
@@ -297,7 +299,7 @@ void gated_scan(const float* q, int ldq, const float* k, int ldk, const float* v
                 const float* beta, int ldb, const float* A_log, const float* dec_bias, float* state,
                 const int32_t* cu_q, const int32_t* state_slot, float* o, int ldo, int R, int heads, int qk_heads,
                 int dk, int dv, int unit, float unit_eps, float q_scale, int decay_kind, float tau,
-                cudaStream_t stream);
+                int longest, cudaStream_t stream);
 
 // qkv f32 rows [q: nh * d | k: nkv * d | v: nkv * dv] (row stride ld).  Every q and k head is divided by its root
 // mean square over d (eps inside the root) and multiplied by qn_w / kn_w (f32 [d], shared by the heads; nullptr: that

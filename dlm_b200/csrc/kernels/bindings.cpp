@@ -145,26 +145,26 @@ PYBIND11_MODULE(_dlm_kernels, m) {
     });
     m.def("ssm_scan", [](u64 xbc, int ldx, u64 dt_raw, int lddt, u64 dt_bias, u64 A_log, u64 D, u64 state, u64 cu_q,
                          u64 state_slot, u64 y, int R, int heads, int P, int N, int groups, u64 fixed_decay,
-                         int silu_inputs, u64 stream) {
+                         int silu_inputs, int longest, u64 stream) {
         dlmk::ssm_scan(ptr<const float>(xbc), ldx, ptr<const float>(dt_raw), lddt, ptr<const float>(dt_bias),
                        ptr<const float>(A_log), ptr<const float>(D), ptr<float>(state), ptr<const int32_t>(cu_q),
                        ptr<const int32_t>(state_slot), ptr<float>(y), R, heads, P, N, groups,
-                       ptr<const float>(fixed_decay), silu_inputs, st(stream));
+                       ptr<const float>(fixed_decay), silu_inputs, longest, st(stream));
     });
     m.def("delta_scan", [](u64 proj, int ld, int off_r, int off_k, int off_v, int off_a, u64 lw, int ldlw, u64 a_bias,
                            u64 state, u64 cu_q, u64 state_slot, u64 o, int R, int heads, int d, float unit_eps,
-                           float decay_coef, u64 stream) {
+                           float decay_coef, int longest, u64 stream) {
         dlmk::delta_scan(ptr<const float>(proj), ld, off_r, off_k, off_v, off_a, ptr<const float>(lw), ldlw,
                          ptr<const float>(a_bias), ptr<float>(state), ptr<const int32_t>(cu_q),
-                         ptr<const int32_t>(state_slot), ptr<float>(o), R, heads, d, unit_eps, decay_coef, st(stream));
+                         ptr<const int32_t>(state_slot), ptr<float>(o), R, heads, d, unit_eps, decay_coef, longest, st(stream));
     });
     m.def("selective_scan", [](u64 x, int ldx, u64 dt_raw, int lddt, u64 bc, int ldbc, u64 z, int ldz, u64 dt_bias, u64 A_log,
                                u64 D, u64 state, u64 cu_q, u64 state_slot, u64 out, int ldo, int R, int inner, int N,
-                               int out_dtype, u64 stream) {
+                               int out_dtype, int longest, u64 stream) {
         dlmk::selective_scan(ptr<const float>(x), ldx, ptr<const float>(dt_raw), lddt, ptr<const float>(bc), ldbc,
                              ptr<const float>(z), ldz, ptr<const float>(dt_bias), ptr<const float>(A_log),
                              ptr<const float>(D), ptr<float>(state), ptr<const int32_t>(cu_q),
-                             ptr<const int32_t>(state_slot), ptr<void>(out), ldo, R, inner, N, out_dtype, st(stream));
+                             ptr<const int32_t>(state_slot), ptr<void>(out), ldo, R, inner, N, out_dtype, longest, st(stream));
     });
     m.def("qk_norm_write", [](u64 qkv, int ld, u64 positions, u64 qn_w, u64 kn_w, float eps, float temp_coef,
                               int temp_every, u64 slots, u64 q_out, u64 k_cache, u64 v_cache, int T, int nh, int nkv,
@@ -222,12 +222,12 @@ PYBIND11_MODULE(_dlm_kernels, m) {
     m.def("gated_scan", [](u64 q, int ldq, u64 k, int ldk, u64 v, int ldv, u64 dec, int ldd, u64 beta, int ldb, u64 A_log,
                            u64 dec_bias, u64 state, u64 cu_q, u64 state_slot, u64 o, int ldo, int R, int heads,
                            int qk_heads, int dk, int dv, int unit, float unit_eps, float q_scale, int decay_kind,
-                           float tau, u64 stream) {
+                           float tau, int longest, u64 stream) {
         dlmk::gated_scan(ptr<const float>(q), ldq, ptr<const float>(k), ldk, ptr<const float>(v), ldv,
                          ptr<const float>(dec), ldd, ptr<const float>(beta), ldb, ptr<const float>(A_log),
                          ptr<const float>(dec_bias), ptr<float>(state), ptr<const int32_t>(cu_q),
                          ptr<const int32_t>(state_slot), ptr<float>(o), ldo, R, heads, qk_heads, dk, dv, unit, unit_eps,
-                         q_scale, decay_kind, tau, st(stream));
+                         q_scale, decay_kind, tau, longest, st(stream));
     });
     m.def("head_norm_rope_write", [](u64 qkv, int ld, u64 positions, u64 qn_w, u64 kn_w, float eps, u64 inv_freq,
                                      int rot_dims, int interleaved, float amplitude, int norm_after, u64 slots,

@@ -578,7 +578,7 @@ void gated_scan(const float* q, int ldq, const float* k, int ldk, const float* v
                 const float* beta, int ldb, const float* A_log, const float* dec_bias, float* state,
                 const int32_t* cu_q, const int32_t* state_slot, float* o, int ldo, int R, int heads, int qk_heads,
                 int dk, int dv, int unit, float unit_eps, float q_scale, int decay_kind, float tau,
-                cudaStream_t stream) {
+                int longest, cudaStream_t stream) {
     if (R <= 0) return;
     DLM_CHECK(dk >= 1 && dk <= 512 && dv >= 1, "gated_scan: key size 1..512");
     DLM_CHECK(qk_heads >= 1 && heads % qk_heads == 0, "gated_scan: heads must be a multiple of the query/key heads");
@@ -588,6 +588,7 @@ void gated_scan(const float* q, int ldq, const float* k, int ldk, const float* v
     const bool delta = beta != nullptr && decay_kind == 0, channel = beta == nullptr && decay_kind == 1 && !unit;
     if (delta || channel) {
         WalkParams w{};
+        w.longest = longest;
         w.q = q; w.ldq = ldq; w.k = k; w.ldk = ldk; w.v = v; w.ldv = ldv; w.dec = dec; w.ldd = ldd;
         w.beta = beta; w.ldb = ldb;
         w.A_log = A_log; w.dec_bias = dec_bias;

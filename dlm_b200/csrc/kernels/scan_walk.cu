@@ -17,8 +17,8 @@
 // themselves that took two to four times as long as the walk.
 //
 // Measured, one request of 2,048 tokens, before (a lane one column, 4-16 rows, everything done by all warps) and now: state space, 64
-// heads of 128 x 64: 900 -> 289 us; retention, 16 heads of 64 x 128, 1,101 tokens: 290 -> 111 us; gated linear attention, 16 heads
-// of 64 x 128: 406 -> 180 us; gated delta rule, 16 heads of 128 x 128: 780 -> 337 us; removal form, 32 heads of 64 x 64: 1,227 -> 316 us.
+// heads of 128 x 64: 824 -> 286 us; retention, 16 heads of 64 x 128: 534 -> 158; gated linear attention, 16 heads of 64 x 128:
+// 577 -> 198; gated delta rule, 16 heads of 128 x 128: 754 -> 352; removal form, 32 heads of 64 x 64: 1,225 -> 305.
 #include "api.h"
 #include "common.cuh"
 #include "scan_walk.h"
@@ -77,6 +77,287 @@ __device__ __forceinline__ float softplus_w(float z) { return z > 20.0f ? z : lo
 constexpr int STAGES = 4, MOST_WALKERS = 4, HELPERS = 8, MOST_WARPS = MOST_WALKERS + HELPERS;
 
 template <int MODE> constexpr int walk_vectors() { return MODE == WALK_REMOVE ? 4 : (MODE == WALK_CHANNEL ? 3 : 2); }
+
+// Row i = 0 .. 7 of a lane: two runs of four, so that a token's vectors come as 16-byte loads.
+template <int RL> __device__ __forceinline__ int row_of(int rlane, int i) { return 4 * rlane + (i & 3) + 4 * RL * (i >> 2); }
+
+// The lane's tile of a state [N, P]: rows (2 i, 2 i + 1) of CPL columns from c0 on.  `vec`: a row's columns come as one access.
+template <int RL, int CPL>
+__device__ __forceinline__ void load_state(const float* st, int N, int P, int rlane, int c0, bool vec, f2 (&s)[4][CPL]) {
+    float raw[8][CPL];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int n = row_of<RL>(rlane, i);
+        const float* src = st + (long long)n * P + c0;
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) raw[i][c] = 0.f;
+        if (n < N) {
+            if (vec && c0 < P) {
+                load_columns(src, raw[i]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < CPL; ++c)
+                    if (c0 + c < P) raw[i][c] = src[c];
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) s[i][c] = pack2(raw[2 * i][c], raw[2 * i + 1][c]);
+}
+
+template <int RL, int CPL>
+__device__ __forceinline__ void store_state(float* st, int N, int P, int rlane, int c0, bool vec, const f2 (&s)[4][CPL]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int n = row_of<RL>(rlane, i);
+        if (n >= N || c0 >= P) continue;
+        float raw[CPL];
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+            const float2 two = unpack2(s[i >> 1][c]);
+            raw[c] = i & 1 ? two.y : two.x;
+        }
+        float* dst = st + (long long)n * P + c0;
+        if (vec) {
+            if (CPL == 4) *reinterpret_cast<float4*>(dst) = make_float4(raw[0], raw[1 % CPL], raw[2 % CPL], raw[3 % CPL]);
+            else *reinterpret_cast<float2*>(dst) = make_float2(raw[0], raw[1 % CPL]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < CPL; ++c)
+                if (c0 + c < P) dst[c] = raw[c];
+        }
+    }
+}
+
+// One token: the lane's tile of the state moves on and the token's output goes to o (the lane's first column there, of which
+// cols_left exist).  sc: the decay and what joins the columns' sums, as prepared.  Fused multiply-adds are spelled out, so that
+// the two kernels that call this give the same bits.
+template <int MODE, int RL, int CPL>
+__device__ __forceinline__ void walk_token(f2 (&s)[4][CPL], const f2 (&q)[4], const f2 (&k)[4], const f2 (&a)[4],
+                                           const f2 (&rr)[4], const float4& sc, const float (&v)[CPL], float dcoef, int rlane,
+                                           int cols_left, float* o) {
+    constexpr bool DELTA = MODE == WALK_DELTA || MODE == WALK_REMOVE;
+    // what joins a column's sum: D v, or the update's share of a read-out taken before the update (u (k . q), or all of `with`)
+    float out[CPL], with[CPL];
+    auto joined = [&](float y, float x) {
+        return MODE == WALK_HEAD ? fmaf(dcoef, x, y) : (MODE == WALK_DELTA ? fmaf(x, sc.z, y) : (MODE == WALK_REMOVE ? y + x : y));
+    };
+    if (!DELTA) {
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+            const float x = MODE == WALK_HEAD ? sc.y * v[c] : v[c];
+            const f2 xx = pack2(x, x);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[i][c] = fma2(a[i], s[i][c], mul2(k[i], xx));
+            f2 acc0 = mul2(s[0][c], q[0]), acc1 = mul2(s[1][c], q[1]);
+            acc0 = fma2(s[2][c], q[2], acc0);
+            acc1 = fma2(s[3][c], q[3], acc1);
+            out[c] = sum2(acc0) + sum2(acc1);
+            with[c] = v[c];
+        }
+    } else {
+        float ks[CPL];
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+            if (MODE == WALK_DELTA) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[i][c] = mul2(s[i][c], a[i]);
+            }
+            f2 k0 = mul2(k[0], s[0][c]), k1 = mul2(k[1], s[1][c]);
+            k0 = fma2(k[2], s[2][c], k0);
+            k1 = fma2(k[3], s[3][c], k1);
+            ks[c] = sum2(k0) + sum2(k1);
+        }
+#pragma unroll
+        for (int o2 = 1; o2 < RL; o2 <<= 1)
+#pragma unroll
+            for (int c = 0; c < CPL; ++c) ks[c] += __shfl_xor_sync(0xffffffffu, ks[c], o2);
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+            f2 q0 = mul2(q[0], s[0][c]), q1 = mul2(q[1], s[1][c]);
+            q0 = fma2(q[2], s[2][c], q0);
+            q1 = fma2(q[3], s[3][c], q1);
+            out[c] = sum2(q0) + sum2(q1);
+            if (MODE == WALK_DELTA) {
+                const float u = sc.y * (v[c] - ks[c]);
+                const f2 uu = pack2(u, u);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[i][c] = fma2(k[i], uu, s[i][c]);
+                with[c] = u;
+            } else {
+                const f2 kk = pack2(ks[c], ks[c]), vv = pack2(v[c], v[c]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[i][c] = fma2(rr[i], kk, fma2(k[i], vv, mul2(a[i], s[i][c])));
+                with[c] = fmaf(v[c], sc.z, -(sc.y * ks[c]));
+            }
+        }
+    }
+    if (RL >= CPL) {
+        // each stage of the sums over a column's row lanes hands half of the columns over, so that CPL columns cost little
+        // more than one; lane `rlane` < CPL ends with column own_c
+        float y;
+        int own_c;
+        if (CPL == 4) {
+            const bool up = rlane & 1, up2 = rlane & 2;
+            float k0 = up ? out[2 % CPL] : out[0], k1 = up ? out[3 % CPL] : out[1 % CPL];
+            k0 += __shfl_xor_sync(0xffffffffu, up ? out[0] : out[2 % CPL], 1);
+            k1 += __shfl_xor_sync(0xffffffffu, up ? out[1 % CPL] : out[3 % CPL], 1);
+            y = (up2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up2 ? k0 : k1, 2);
+            own_c = (rlane & 1) << 1 | ((rlane >> 1) & 1);
+        } else {
+            const bool up = rlane & 1;
+            y = (up ? out[1 % CPL] : out[0]) + __shfl_xor_sync(0xffffffffu, up ? out[0] : out[1 % CPL], 1);
+            own_c = rlane & 1;
+        }
+#pragma unroll
+        for (int o2 = CPL; o2 < RL; o2 <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o2);
+        y = joined(y, CPL == 4 ? (own_c & 2 ? (own_c & 1 ? with[3 % CPL] : with[2 % CPL]) : (own_c & 1 ? with[1 % CPL] : with[0]))
+                               : (own_c ? with[1 % CPL] : with[0]));
+        if (rlane < CPL && own_c < cols_left) o[own_c] = y;
+    } else {
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+            float y = out[c];
+#pragma unroll
+            for (int x = 1; x < RL; x <<= 1) y += __shfl_xor_sync(0xffffffffu, y, x);
+            if (rlane == 0 && c < cols_left) o[c] = joined(y, with[c]);
+        }
+    }
+}
+
+// x[i] <- f(x[i], row of i) for the lane's eight rows.  The 32 / RL column lanes of a row group hold the same x, so each works out
+// a share and hands it round.
+template <int RL, typename F>
+__device__ __forceinline__ void each_row(float (&x)[8], int lane, F f) {
+    constexpr int G = 32 / RL < 8 ? 32 / RL : 8, E = 8 / G;
+    const int rlane = lane & (RL - 1), g = (lane / RL) % G;
+    float y[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        float v = x[e];
+#pragma unroll
+        for (int j = 1; j < G; ++j) v = g == j ? x[j * E + e] : v;
+        y[e] = f(v, row_of<RL>(rlane, g * E + e));
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = G == 1 ? y[i % E] : __shfl_sync(0xffffffffu, y[i % E], rlane + RL * (i / E));
+}
+
+// Steps whose requests all have few tokens: no ring and no helpers.  Block = (head, request, a run of columns); every warp walks,
+// loads a token's raw values for its lanes' rows and columns and prepares them in registers, in the order of operations (and of
+// the sums over N) of the helpers of the kernel below.  What bounds such a step is the latency of one block where there are
+// few and the states' traffic where there are many: the kernel below has one block a multiprocessor and its ring to fill first.
+// Measured, 64 requests of one token, in the kernel below and here: state space, 64 heads of 128 x 64: 159 and 91 us; retention,
+// 16 heads of 64 x 128: 34 and 21; gated delta rule, 16 heads of 128 x 128: 87 and 48; removal form, 32 heads of 64 x 64: 54 and 26.
+template <int MODE, int RL, int CPL>
+__global__ void __launch_bounds__(32 * MOST_WALKERS, 3) scan_few_kernel(WalkParams p) {
+    dep_wait();           // nothing is read or written before the kernels before this one have ended
+    constexpr bool CHANNEL = MODE == WALK_CHANNEL || MODE == WALK_REMOVE;
+    const int h = blockIdx.x, r = blockIdx.y, lane = threadIdx.x & 31, rlane = lane & (RL - 1);
+    const int first = (blockIdx.z * p.walkers + (int)(threadIdx.x >> 5)) * (32 / RL * CPL), c0 = first + (lane / RL) * CPL;
+    const int N = p.N, P = p.P, hq = h / p.q_div;
+    if (first >= P) return;
+    // (what does not depend on another load is asked for before anything is waited for)
+    const bool fixed = MODE == WALK_HEAD && p.fixed_decay != nullptr, per_head = (MODE == WALK_HEAD && !fixed) || MODE == WALK_DELTA;
+    const int t0 = p.cu_q[r], t1 = p.cu_q[r + 1], slot = p.state_slot[r];
+    const float A_log = per_head ? p.A_log[h] : 0.f, fixed_a = fixed ? p.fixed_decay[h] : 0.f;
+    const float bias = per_head && p.dec_bias != nullptr ? p.dec_bias[h] : 0.f;
+    const float dcoef = MODE == WALK_HEAD && p.D != nullptr ? p.D[h] : 0.f;
+    if (t0 >= t1) return;
+    float* st = p.state + ((long long)slot * p.heads + h) * (long long)N * P;
+    f2 s[4][CPL];
+    load_state<RL, CPL>(st, N, P, rlane, c0, p.state_vec != 0, s);
+    const float rate = per_head ? -expf(A_log) : 0.f;
+
+    auto rows = [&](const float* src, float (&x)[8]) {     // the lane's entries of a vector of N, zeros beyond
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const int at = 4 * rlane + 4 * RL * g;
+            if (p.wide) {
+                const float4 v = at < N ? *reinterpret_cast<const float4*>(src + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[4 * g] = v.x; x[4 * g + 1] = v.y; x[4 * g + 2] = v.z; x[4 * g + 3] = v.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[4 * g + e] = at + e < N ? src[at + e] : 0.f;
+            }
+        }
+    };
+    // sum over N of x y, as the lanes of a helper add it up: one chain a four (RL = 32: one for both fours), then pairs of
+    // neighbouring lanes, pairs of pairs, ...
+    auto dot = [&](const float (&x)[8], const float (&y)[8]) {
+        float part[2] = {0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[RL == 32 ? 0 : i >> 2] = fmaf(x[i], y[i], part[RL == 32 ? 0 : i >> 2]);
+#pragma unroll
+        for (int o = 1; o < RL; o <<= 1) {
+            part[0] += __shfl_xor_sync(0xffffffffu, part[0], o);
+            if (RL < 32) part[1] += __shfl_xor_sync(0xffffffffu, part[1], o);
+        }
+        return RL == 32 ? part[0] : part[0] + part[1];
+    };
+    for (long long t = t0; t < t1; ++t) {
+        float q[8], k[8], a[8], rr[8], v[CPL];
+        float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
+        rows(p.q + t * p.ldq + (long long)hq * N, q);
+        rows(p.k + t * p.ldk + (long long)hq * N, k);
+        if (CHANNEL) rows(p.dec + t * p.ldd + (long long)h * N, a);
+        if (MODE == WALK_REMOVE) rows(p.rate + t * p.ldr + (long long)h * N, rr);
+        const float* src = p.v + t * p.ldv + (long long)h * P + c0;
+        if (p.wide && c0 < P) {
+            load_columns(src, v);
+        } else {
+#pragma unroll
+            for (int c = 0; c < CPL; ++c) v[c] = c0 + c < P ? src[c] : 0.f;
+        }
+        if (MODE == WALK_HEAD) {
+            const float dt = fixed ? 1.0f : softplus_w(p.dec[t * p.ldd + h] + bias);
+            sc.x = fixed ? fixed_a : expf(rate * dt);
+            sc.y = dt;
+            if (p.silu_inputs) {
+                each_row<RL>(q, lane, [](float x, int) { return silu_f(x); });
+                each_row<RL>(k, lane, [](float x, int) { return silu_f(x); });
+#pragma unroll
+                for (int c = 0; c < CPL; ++c) v[c] = silu_f(v[c]);
+            }
+        } else if (MODE == WALK_CHANNEL) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[i] *= p.q_scale;
+            each_row<RL>(a, lane, [&](float x, int) { return expf(-softplus_w(-x) * p.inv_tau); });
+        } else if (MODE == WALK_DELTA) {
+            const float qq = dot(q, q), kk = dot(k, k), qk = dot(q, k);
+            const float fq = p.unit ? p.q_scale * (1.0f / sqrtf(qq + p.unit_eps)) : p.q_scale;
+            const float fk = p.unit ? 1.0f / sqrtf(kk + p.unit_eps) : 1.0f;
+            sc.x = expf(rate * softplus_w(p.dec[t * p.ldd + h] + bias));
+            sc.y = sigmoid_w(p.beta[t * p.ldb + h]);
+            sc.z = qk * (fq * fk);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { q[i] *= fq; k[i] *= fk; }
+        } else {
+            each_row<RL>(a, lane, [&](float x, int n) { return n < N ? expf(-p.decay_coef * sigmoid_w(x)) : 0.f; });
+            each_row<RL>(rr, lane, [&](float x, int n) { return n < N ? sigmoid_w(x + p.rate_bias[(long long)h * N + n]) : 0.f; });
+#pragma unroll
+            for (int i = 0; i < 8; ++i) rr[i] *= k[i];
+            const float kk = dot(k, k), qk = dot(q, k), qr = dot(q, rr);
+            const float inv = 1.0f / sqrtf(kk + p.unit_eps);
+            sc.y = qr * inv * inv;
+            sc.z = qk;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { q[i] *= a[i]; rr[i] = -rr[i] * inv * inv; }
+        }
+        f2 q2[4], k2[4], a2[4], r2[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            q2[i] = pack2(q[2 * i], q[2 * i + 1]);
+            k2[i] = pack2(k[2 * i], k[2 * i + 1]);
+            a2[i] = CHANNEL ? pack2(a[2 * i], a[2 * i + 1]) : pack2(sc.x, sc.x);
+            if (MODE == WALK_REMOVE) r2[i] = pack2(rr[2 * i], rr[2 * i + 1]);
+        }
+        walk_token<MODE, RL, CPL>(s, q2, k2, a2, r2, sc, v, dcoef, rlane, P - c0, p.o + t * p.ldo + (long long)h * P + c0);
+    }
+    store_state<RL, CPL>(st, N, P, rlane, c0, p.state_vec != 0, s);
+}
 
 // RL: lanes that share a column's rows (N <= 8 RL).  Block = (head, request, a run of columns); the first p.walkers warps walk,
 // CPL 32 / RL columns each, the others help.
@@ -270,53 +551,8 @@ __global__ void __launch_bounds__(32 * MOST_WARPS, 1) scan_walk_kernel(WalkParam
     const int rlane = lane & (RL - 1), c_local = warp * CW + (lane / RL) * CPL, c0 = p0 + c_local;
     const float dcoef = MODE == WALK_HEAD && p.D != nullptr ? p.D[h] : 0.f;
     float* st = p.state + ((long long)p.state_slot[r] * p.heads + h) * (long long)N * P;
-    auto row_of = [&](int i) { return 4 * rlane + (i & 3) + 4 * RL * (i >> 2); };     // i = 0 .. 7
-    const bool vec = p.state_vec != 0;
-    f2 s[4][CPL];                                          // rows (2 i, 2 i + 1) of the lane's columns
-    {
-        float raw[8][CPL];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int n = row_of(i);
-            const float* src = st + (long long)n * P + c0;
-#pragma unroll
-            for (int c = 0; c < CPL; ++c) raw[i][c] = 0.f;
-            if (n < N) {
-                if (vec && c0 < P) {
-                    load_columns(src, raw[i]);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < CPL; ++c)
-                        if (c0 + c < P) raw[i][c] = src[c];
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int c = 0; c < CPL; ++c) s[i][c] = pack2(raw[2 * i][c], raw[2 * i + 1][c]);
-    }
-
-    // sums over a column's row lanes: with at least CPL of them each stage hands half of the columns over, so that CPL
-    // columns cost little more than one; lane `rlane` < CPL ends with column own_c
-    const int own_c = CPL == 4 ? ((rlane & 1) << 1 | ((rlane >> 1) & 1)) : (rlane & 1);
-    auto reduce_columns = [&](const float (&a)[CPL]) {
-        float v;
-        if (CPL == 4) {
-            const bool up = rlane & 1;
-            float k0 = up ? a[2 % CPL] : a[0], k1 = up ? a[3 % CPL] : a[1 % CPL];
-            k0 += __shfl_xor_sync(0xffffffffu, up ? a[0] : a[2 % CPL], 1);
-            k1 += __shfl_xor_sync(0xffffffffu, up ? a[1 % CPL] : a[3 % CPL], 1);
-            const bool up2 = rlane & 2;
-            v = (up2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up2 ? k0 : k1, 2);
-        } else {
-            const bool up = rlane & 1;
-            v = (up ? a[1 % CPL] : a[0]) + __shfl_xor_sync(0xffffffffu, up ? a[0] : a[1 % CPL], 1);
-        }
-#pragma unroll
-        for (int o = CPL; o < RL; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        return v;
-    };
+    f2 s[4][CPL];
+    load_state<RL, CPL>(st, N, P, rlane, c0, p.state_vec != 0, s);
 
     __syncthreads();
     for (int tile = 0; tile < n_tiles; ++tile) {
@@ -347,96 +583,12 @@ __global__ void __launch_bounds__(32 * MOST_WARPS, 1) scan_walk_kernel(WalkParam
             }
             float v[CPL];
             load_columns(row + off_v + c_local, v);
-            // `add`: what joins a column's sum: D v, or the update's share of a read-out taken before the update
-            float out[CPL], add[CPL];
-            if (!DELTA) {
-#pragma unroll
-                for (int c = 0; c < CPL; ++c) {
-                    const float x = MODE == WALK_HEAD ? sc.y * v[c] : v[c];
-                    const f2 xx = pack2(x, x);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) s[i][c] = fma2(a[i], s[i][c], mul2(k[i], xx));
-                    f2 acc0 = mul2(s[0][c], q[0]), acc1 = mul2(s[1][c], q[1]);
-                    acc0 = fma2(s[2][c], q[2], acc0);
-                    acc1 = fma2(s[3][c], q[3], acc1);
-                    out[c] = sum2(acc0) + sum2(acc1);
-                    add[c] = MODE == WALK_HEAD ? dcoef * v[c] : 0.f;
-                }
-            } else {
-                float ks[CPL];
-#pragma unroll
-                for (int c = 0; c < CPL; ++c) {
-                    if (MODE == WALK_DELTA) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) s[i][c] = mul2(s[i][c], a[i]);
-                    }
-                    f2 k0 = mul2(k[0], s[0][c]), k1 = mul2(k[1], s[1][c]);
-                    k0 = fma2(k[2], s[2][c], k0);
-                    k1 = fma2(k[3], s[3][c], k1);
-                    ks[c] = sum2(k0) + sum2(k1);
-                }
-#pragma unroll
-                for (int o = 1; o < RL; o <<= 1)
-#pragma unroll
-                    for (int c = 0; c < CPL; ++c) ks[c] += __shfl_xor_sync(0xffffffffu, ks[c], o);
-#pragma unroll
-                for (int c = 0; c < CPL; ++c) {
-                    f2 q0 = mul2(q[0], s[0][c]), q1 = mul2(q[1], s[1][c]);
-                    q0 = fma2(q[2], s[2][c], q0);
-                    q1 = fma2(q[3], s[3][c], q1);
-                    out[c] = sum2(q0) + sum2(q1);
-                    if (MODE == WALK_DELTA) {
-                        const float u = sc.y * (v[c] - ks[c]);
-                        const f2 uu = pack2(u, u);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) s[i][c] = fma2(k[i], uu, s[i][c]);
-                        add[c] = u * sc.z;
-                    } else {
-                        const f2 kk = pack2(ks[c], ks[c]), vv = pack2(v[c], v[c]);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) s[i][c] = fma2(rr[i], kk, fma2(k[i], vv, mul2(a[i], s[i][c])));
-                        add[c] = fmaf(v[c], sc.z, -sc.y * ks[c]);
-                    }
-                }
-            }
-            float* o = p.o + (long long)(first + tok) * p.ldo + (long long)h * P + c0;
-            if (RL >= CPL) {
-                float y = reduce_columns(out);
-                if (MODE != WALK_CHANNEL) y += CPL == 4 ? (own_c & 2 ? (own_c & 1 ? add[3 % CPL] : add[2 % CPL]) : (own_c & 1 ? add[1 % CPL] : add[0]))
-                                                        : (own_c ? add[1 % CPL] : add[0]);
-                if (rlane < CPL && c0 + own_c < P) o[own_c] = y;
-            } else {
-#pragma unroll
-                for (int c = 0; c < CPL; ++c) {
-                    float y = out[c];
-#pragma unroll
-                    for (int x = 1; x < RL; x <<= 1) y += __shfl_xor_sync(0xffffffffu, y, x);
-                    if (rlane == 0 && c0 + c < P) o[c] = y + add[c];
-                }
-            }
+            walk_token<MODE, RL, CPL>(s, q, k, a, rr, sc, v, dcoef, rlane, P - c0,
+                                      p.o + (long long)(first + tok) * p.ldo + (long long)h * P + c0);
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int n = row_of(i);
-        if (n >= N || c0 >= P) continue;
-        float raw[CPL];
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) {
-            const float2 two = unpack2(s[i >> 1][c]);
-            raw[c] = i & 1 ? two.y : two.x;
-        }
-        float* dst = st + (long long)n * P + c0;
-        if (vec) {
-            if (CPL == 4) *reinterpret_cast<float4*>(dst) = make_float4(raw[0], raw[1 % CPL], raw[2 % CPL], raw[3 % CPL]);
-            else *reinterpret_cast<float2*>(dst) = make_float2(raw[0], raw[1 % CPL]);
-        } else {
-#pragma unroll
-            for (int c = 0; c < CPL; ++c)
-                if (c0 + c < P) dst[c] = raw[c];
-        }
-    }
+    store_state<RL, CPL>(st, N, P, rlane, c0, p.state_vec != 0, s);
 }
 
 template <int MODE, int RL, int CPL>
@@ -446,21 +598,29 @@ void launch_walk(WalkParams p, int R, int walkers, cudaStream_t stream) {
     const int row = walk_vectors<MODE>() * 8 * RL + ((cols + 3) & ~3) + 4;
     p.walkers = walkers;
     p.state_vec = p.P % CPL == 0 && reinterpret_cast<uintptr_t>(p.state) % (CPL * sizeof(float)) == 0 ? 1 : 0;
+    const dim3 grid(p.heads, R, (p.P + cols - 1) / cols);
+    // One token a request, or two or three where the ring's kernel would need more than one wave (64 requests of three tokens,
+    // gated delta rule, 16 heads of 128 x 128: 101 us there, 72 here; with four tokens the chain of loads a token costs as much
+    // as it saves: 32 requests, gated linear attention, 16 heads of 64 x 128: 23 and 27).
+    if (p.longest == 1 || (p.longest >= 1 && p.longest <= 3 && (long long)grid.x * grid.y * grid.z > sm_count())) {
+        scan_few_kernel<MODE, RL, CPL><<<grid, 32 * walkers, 0, stream>>>(p);
+        return;
+    }
     p.wide_v = p.wide && cols % 4 == 0 ? 1 : 0;              // (a block's first column is a multiple of `cols`)
     p.tile = 16;
     while (p.tile > 1 && (size_t)STAGES * p.tile * row * sizeof(float) > 150 * 1024) p.tile /= 2;
     const size_t smem = (size_t)STAGES * p.tile * row * sizeof(float);
     auto kern = scan_walk_kernel<MODE, RL, CPL>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<dim3(p.heads, R, (p.P + cols - 1) / cols), 32 * (walkers + HELPERS), smem, stream>>>(p);
+    kern<<<grid, 32 * (walkers + HELPERS), smem, stream>>>(p);
 }
 
 template <int MODE, int RL>
 void launch_rl(const WalkParams& p, int R, cudaStream_t stream) {
     constexpr int CL = 32 / RL;
     auto blocks = [&](int cpl, int walkers) { return (long long)p.heads * R * ((p.P + walkers * CL * cpl - 1) / (walkers * CL * cpl)); };
-    // Four columns a lane where that still leaves four warps a multiprocessor (64 heads of 128 x 64, 2,048 tokens: 289 us
-    // against 401 with two), two otherwise (32 heads of 64 x 64: 316 against 444; 16 heads of 128 x 128: 337 against 421).
+    // Four columns a lane where that still leaves three warps a multiprocessor (64 heads of 128 x 64, 2,048 tokens, 3.5 warps:
+    // 289 us against 401 with two), two otherwise (32 heads of 64 x 64: 316 against 444; 16 heads of 128 x 128: 337 against 421).
     const int cpl = blocks(4, 1) >= 3LL * sm_count() ? 4 : 2;
     // Four walkers a block, which then share one preparation; two where there would be a block for less than every other
     // multiprocessor (32 heads of 64 x 64: 316 us against 346; 16 heads of 64 x 128 with a decay per channel: 180 against 212).

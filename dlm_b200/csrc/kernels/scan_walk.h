@@ -25,6 +25,7 @@ struct WalkParams {
     int heads, q_div, N, P;
     int silu_inputs, unit;
     float unit_eps, q_scale, inv_tau, decay_coef;
+    int longest;                         // tokens of the step's longest request, or a bound of it; 0: not known
     int wide, wide_v, state_vec, walkers, tile;      // filled in by scan_walk: 16-byte copies are possible (of the vectors, of
                                          // v), a lane's columns of the state come as one access; warps that walk; tokens a tile
 };

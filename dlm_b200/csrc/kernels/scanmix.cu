@@ -41,7 +41,7 @@ template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("c
 // 2^(dt A log2 e) with A log2 e kept in registers; a channel's sum is added per lane in a fixed order, then by shuffles.
 // Bound by the instructions issued per token.  Measured (4,096 channels of 16 states, requests of 1,101, 652 and 203 tokens): 368 us
 // with two states a lane, a shared-memory store per token and three phases a tile, 343 us with four helpers that prepared four
-// neighbouring channels a lane, about 143 us now.
+// neighbouring channels a lane, about 143 us with eight.  (One request of 2,048 tokens: 439 us then, 197 now.)
 constexpr int SCAN_WALKERS = 4, SCAN_HELPERS = 8, SCAN_STAGES = 4;
 
 typedef unsigned long long f2;        // two floats, the lower one first
@@ -72,13 +72,134 @@ __device__ __forceinline__ float ex2_ftz(float x) {
     return y;
 }
 
+// One token of a channel: the lane's eight states move on; returns the sum of s C over the channel's states (in every lane).
+template <int PARTS>
+__device__ __forceinline__ float selective_token(f2 (&s)[4], const f2 (&a2)[4], const f2 (&bb)[4], const f2 (&cc)[4], float dt,
+                                                 float xv) {
+    const f2 dt2 = pack2(dt, dt), dx2 = pack2(dt * xv, dt * xv);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 w = unpack2(mul2(dt2, a2[i]));
+        s[i] = fma2(pack2(ex2_ftz(w.x), ex2_ftz(w.y)), s[i], mul2(dx2, bb[i]));
+    }
+    f2 u = mul2(s[0], cc[0]), v = mul2(s[1], cc[1]);
+    u = fma2(s[2], cc[2], u);
+    v = fma2(s[3], cc[3], v);
+    const float2 uu = unpack2(u), vv = unpack2(v);
+    float sum = (uu.x + uu.y) + (vv.x + vv.y);
+#pragma unroll
+    for (int o = 1; o < PARTS; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+}
+
+// A prepared tile of n tokens: rows of rl floats [B | C | dt | x | gate], o the channel's output of the first.
+template <int PARTS, typename TOut>
+__device__ __forceinline__ void selective_tile(const float* buf, int n, int rl, int cp, int part, int col, bool live, f2 (&s)[4],
+                                               const f2 (&a2)[4], float d_c, TOut* o, int ldo) {
+    constexpr int NP = 8 * PARTS;
+#pragma unroll 4
+    for (int tok = 0; tok < n; ++tok) {
+        const float* row = buf + (size_t)tok * rl;
+        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(row + 8 * part);
+        const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(row + 8 * part + 4);
+        const ulonglong2 e0 = *reinterpret_cast<const ulonglong2*>(row + NP + 8 * part);
+        const ulonglong2 e1 = *reinterpret_cast<const ulonglong2*>(row + NP + 8 * part + 4);
+        const float dt = row[2 * NP + col], xv = row[2 * NP + cp + col], gate = row[2 * NP + 2 * cp + col];
+        const f2 bb[4] = {b0.x, b0.y, b1.x, b1.y}, cc[4] = {e0.x, e0.y, e1.x, e1.y};
+        const float sum = selective_token<PARTS>(s, a2, bb, cc, dt, xv);
+        if (live && part == 0) o[(long long)tok * ldo] = from_f32<TOut>(fmaf(d_c, xv, sum) * gate);
+    }
+}
+
+struct SelectiveArgs {
+    const float* x; int ldx;
+    const float* dt_raw; int lddt;
+    const float* bc; int ldbc;
+    const float* z; int ldz;
+    const float* dt_bias; const float* A_log; const float* D;
+    float* state;
+    const int32_t* cu_q; const int32_t* state_slot;
+    int ldo, inner, N, wide_bc;          // wide_bc: the eights of a token's B and C start on 16-byte boundaries
+};
+
+// The lane's eight states of channel c and their A log2 e (zeros beyond N, and in lanes without a channel).
+template <int PARTS>
+__device__ __forceinline__ void selective_load(const SelectiveArgs& p, const float* st, int c, int part, bool live, f2 (&s)[4],
+                                               f2 (&a2)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float sv[2], av[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int n = 8 * part + 2 * i + e;
+            const bool ok = live && n < p.N;
+            sv[e] = ok ? st[n] : 0.f;
+            av[e] = ok ? -expf(p.A_log[(long long)c * p.N + n]) * 1.4426950408889634f : 0.f;
+        }
+        s[i] = pack2(sv[0], sv[1]);
+        a2[i] = pack2(av[0], av[1]);
+    }
+}
+__device__ __forceinline__ void selective_store(float* st, int N, int part, bool live, const f2 (&s)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 two = unpack2(s[i]);
+        const int n = 8 * part + 2 * i;
+        if (live && n < N) st[n] = two.x;
+        if (live && n + 1 < N) st[n + 1] = two.y;
+    }
+}
+
+// Steps whose requests all have few tokens: no ring and no helpers.  Block = (a run of channels, request); every warp walks and
+// loads what its channels and their states need of a token.  (64 requests of one token, 4,096 channels of 16 states: 72 us in
+// the kernel below, whose blocks have a multiprocessor to themselves, 21 here; four tokens each: 41 and 17 for 32 requests.)
+template <int PARTS, typename TOut>
+__global__ void __launch_bounds__(32 * SCAN_WALKERS) selective_few_kernel(SelectiveArgs p, TOut* out) {
+    dep_wait();          // nothing is read or written before the kernels before this one have ended
+    const int r = blockIdx.y, lane = threadIdx.x & 31, part = lane % PARTS;
+    const int c = (blockIdx.x * (blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * (32 / PARTS) + lane / PARTS;
+    const bool live = c < p.inner;
+    const int N = p.N, ch = live ? c : 0;
+    const int t0 = p.cu_q[r], t1 = p.cu_q[r + 1], slot = p.state_slot[r];
+    const float d_c = p.D[ch], bias = p.dt_bias[ch];
+    if (t0 >= t1) return;
+    float* st = p.state + ((long long)slot * p.inner + ch) * N;
+    f2 s[4], a2[4];
+    selective_load<PARTS>(p, st, c, part, live, s, a2);
+    for (long long t = t0; t < t1; ++t) {
+        const float* row = p.bc + t * p.ldbc;
+        f2 bb[4], cc[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            f2 (&dst)[4] = h == 0 ? bb : cc;
+            const float* src = row + h * N + 8 * part;
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                float v[4];
+                if (p.wide_bc) {
+                    const float4 w = 8 * part + 4 * g < N ? *reinterpret_cast<const float4*>(src + 4 * g)
+                                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) v[e] = 8 * part + 4 * g + e < N ? src[4 * g + e] : 0.f;
+                }
+                dst[2 * g] = pack2(v[0], v[1]);
+                dst[2 * g + 1] = pack2(v[2], v[3]);
+            }
+        }
+        const float dt = softplus_f(p.dt_raw[t * p.lddt + ch] + bias), xv = p.x[t * p.ldx + ch], gate = silu_f(p.z[t * p.ldz + ch]);
+        const float sum = selective_token<PARTS>(s, a2, bb, cc, dt, xv);
+        if (live && part == 0) out[t * p.ldo + c] = from_f32<TOut>(fmaf(d_c, xv, sum) * gate);
+    }
+    selective_store(st, N, part, live, s);
+}
+
 template <int PARTS, typename TOut>
 __global__ void __launch_bounds__(32 * (SCAN_WALKERS + SCAN_HELPERS), 1)
-selective_scan_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ dt_raw, int lddt,
-                      const float* __restrict__ bc, int ldbc, const float* __restrict__ z, int ldz,
-                      const float* __restrict__ dt_bias, const float* __restrict__ A_log, const float* __restrict__ D,
-                      float* state, const int32_t* __restrict__ cu_q, const int32_t* __restrict__ state_slot, TOut* out,
-                      int ldo, int inner, int N, int walkers, int tile_tokens, int wide) {
+selective_scan_kernel(SelectiveArgs p, TOut* out, int walkers, int tile_tokens, int wide) {
+    const float* x = p.x; const float* dt_raw = p.dt_raw; const float* bc = p.bc; const float* z = p.z;
+    const int ldx = p.ldx, lddt = p.lddt, ldbc = p.ldbc, ldz = p.ldz, inner = p.inner, N = p.N;
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     constexpr int NP = 8 * PARTS, CW = 32 / PARTS;        // states as stored; channels of a warp
     extern __shared__ __align__(16) float sm[];           // [STAGES][tile][B: NP | C: NP | dt | x | gate: cp each]
@@ -86,7 +207,7 @@ selective_scan_kernel(const float* __restrict__ x, int ldx, const float* __restr
     const int chans = walkers * CW, cp = (chans + 3) & ~3, rl = 2 * NP + 3 * cp;
     const int c0 = blockIdx.x * chans, nch = min(chans, inner - c0);
     const int r = blockIdx.y;
-    const int t0 = cu_q[r], t1 = cu_q[r + 1];
+    const int t0 = p.cu_q[r], t1 = p.cu_q[r + 1];
     const int n_tiles = (t1 - t0 + tile_tokens - 1) / tile_tokens;
 
     if (warp >= walkers) {
@@ -135,7 +256,7 @@ selective_scan_kernel(const float* __restrict__ x, int ldx, const float* __restr
                 float* dt = buf + (size_t)tok * rl + 2 * NP;
                 float* gate = dt + 2 * cp;
                 for (int i = lane; i < nch; i += 32) {
-                    dt[i] = softplus_f(dt[i] + dt_bias[c0 + i]);
+                    dt[i] = softplus_f(dt[i] + p.dt_bias[c0 + i]);
                     gate[i] = silu_f(gate[i]);
                 }
             }
@@ -156,59 +277,19 @@ selective_scan_kernel(const float* __restrict__ x, int ldx, const float* __restr
 
     const int part = lane % PARTS, col = warp * CW + lane / PARTS, c = c0 + col;
     const bool live = c < inner;
-    float* st = state + ((long long)state_slot[r] * inner + (live ? c : 0)) * N;
+    float* st = p.state + ((long long)p.state_slot[r] * inner + (live ? c : 0)) * N;
     f2 s[4], a2[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float sv[2], av[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int n = 8 * part + 2 * i + e;
-            const bool ok = live && n < N;
-            sv[e] = ok ? st[n] : 0.f;
-            av[e] = ok ? -expf(A_log[(long long)c * N + n]) * 1.4426950408889634f : 0.f;
-        }
-        s[i] = pack2(sv[0], sv[1]);
-        a2[i] = pack2(av[0], av[1]);
-    }
-    const float d_c = live ? D[c] : 0.f;
+    selective_load<PARTS>(p, st, c, part, live, s, a2);
+    const float d_c = live ? p.D[c] : 0.f;
     __syncthreads();
     for (int k = 0; k < n_tiles; ++k) {
         const float* buf = sm + (size_t)(k % SCAN_STAGES) * tile_tokens * rl;
         const int first = t0 + k * tile_tokens, n = min(tile_tokens, t1 - first);
-#pragma unroll 4
-        for (int tok = 0; tok < n; ++tok) {
-            const float* row = buf + (size_t)tok * rl;
-            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(row + 8 * part);
-            const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(row + 8 * part + 4);
-            const ulonglong2 e0 = *reinterpret_cast<const ulonglong2*>(row + NP + 8 * part);
-            const ulonglong2 e1 = *reinterpret_cast<const ulonglong2*>(row + NP + 8 * part + 4);
-            const float dt = row[2 * NP + col], xv = row[2 * NP + cp + col], gate = row[2 * NP + 2 * cp + col];
-            const f2 bb[4] = {b0.x, b0.y, b1.x, b1.y}, cc[4] = {e0.x, e0.y, e1.x, e1.y};
-            const f2 dt2 = pack2(dt, dt), dx2 = pack2(dt * xv, dt * xv);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 w = unpack2(mul2(dt2, a2[i]));
-                s[i] = fma2(pack2(ex2_ftz(w.x), ex2_ftz(w.y)), s[i], mul2(dx2, bb[i]));
-            }
-            f2 u = mul2(s[0], cc[0]), v = mul2(s[1], cc[1]);
-            u = fma2(s[2], cc[2], u);
-            v = fma2(s[3], cc[3], v);
-            const float2 uu = unpack2(u), vv = unpack2(v);
-            float sum = (uu.x + uu.y) + (vv.x + vv.y);
-#pragma unroll
-            for (int o = 1; o < PARTS; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (live && part == 0) out[(long long)(first + tok) * ldo + c] = from_f32<TOut>(fmaf(d_c, xv, sum) * gate);
-        }
+        TOut* o = out + (long long)first * p.ldo + c;
+        selective_tile<PARTS>(buf, n, rl, cp, part, col, live, s, a2, d_c, o, p.ldo);
         __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 two = unpack2(s[i]);
-        const int n = 8 * part + 2 * i;
-        if (live && n < N) st[n] = two.x;
-        if (live && n + 1 < N) st[n + 1] = two.y;
-    }
+    selective_store(st, N, part, live, s);
 }
 
 // ------------------------------------------------- whole-projection norms, temperature, cache write
@@ -376,7 +457,7 @@ __global__ void concat_rows_kernel(const float* a, const float* b, T* out, int H
 void selective_scan(const float* x, int ldx, const float* dt_raw, int lddt, const float* bc, int ldbc, const float* z,
                     int ldz, const float* dt_bias, const float* A_log, const float* D, float* state,
                     const int32_t* cu_q, const int32_t* state_slot, void* out, int ldo, int R, int inner, int N,
-                    int out_dtype, cudaStream_t stream) {
+                    int out_dtype, int longest, cudaStream_t stream) {
     if (R <= 0 || inner <= 0) return;
     DLM_CHECK(N >= 1 && N <= 256, "selective_scan: state size 1..256");
     int parts = 1;
@@ -394,13 +475,20 @@ void selective_scan(const float* x, int ldx, const float* dt_raw, int lddt, cons
     const int wide = (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dt_raw) | reinterpret_cast<uintptr_t>(bc) |
                         reinterpret_cast<uintptr_t>(z)) & 15) == 0 && ldx % 4 == 0 && lddt % 4 == 0 && ldbc % 4 == 0 &&
                       ldz % 4 == 0 && N % 4 == 0 && chans % 4 == 0 && inner % 4 == 0) ? 1 : 0;
+    const int wide_bc = (reinterpret_cast<uintptr_t>(bc) & 15) == 0 && ldbc % 4 == 0 && N % 4 == 0 ? 1 : 0;
+    const SelectiveArgs args{x, ldx, dt_raw, lddt, bc, ldbc, z, ldz, dt_bias, A_log, D, state, cu_q, state_slot, ldo, inner, N, wide_bc};
+    // One token a request, or up to four where the ring's kernel would need more than one wave of blocks
+    const bool few = longest == 1 || (longest >= 1 && longest <= 4 && (long long)grid.x * grid.y > sm_count());
 #define DLM_SEL(PARTS, TOUT)                                                                                         \
     do {                                                                                                             \
+        if (few) {                                                                                                   \
+            selective_few_kernel<PARTS, TOUT><<<grid, 32 * walkers, 0, stream>>>(args, static_cast<TOUT*>(out));     \
+            break;                                                                                                   \
+        }                                                                                                            \
         auto kern = selective_scan_kernel<PARTS, TOUT>;                                                              \
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
-        kern<<<grid, 32 * (walkers + SCAN_HELPERS), smem, stream>>>(                                                 \
-            x, ldx, dt_raw, lddt, bc, ldbc, z, ldz, dt_bias, A_log, D, state, cu_q, state_slot,                      \
-            static_cast<TOUT*>(out), ldo, inner, N, walkers, tile, wide);                                            \
+        kern<<<grid, 32 * (walkers + SCAN_HELPERS), smem, stream>>>(args, static_cast<TOUT*>(out), walkers, tile,    \
+                                                                    wide);                                           \
     } while (0)
 #define DLM_SEL_T(PARTS)                                                                   \
     do {                                                                                   \

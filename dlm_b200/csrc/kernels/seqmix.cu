@@ -1019,7 +1019,7 @@ void gated_rmsnorm(const float* y, int ldy, const float* gate, int ldg, const fl
 
 void ssm_scan(const float* xbc, int ldx, const float* dt_raw, int lddt, const float* dt_bias, const float* A_log,
               const float* D, float* state, const int32_t* cu_q, const int32_t* state_slot, float* y, int R, int heads,
-              int P, int N, int groups, const float* fixed_decay, int silu_inputs, cudaStream_t stream) {
+              int P, int N, int groups, const float* fixed_decay, int silu_inputs, int longest, cudaStream_t stream) {
     if (R <= 0) return;
     DLM_CHECK(fixed_decay != nullptr || (dt_raw != nullptr && dt_bias != nullptr && A_log != nullptr && D != nullptr),
               "ssm_scan: without fixed decays the step sizes, their bias, A_log and D are needed");
@@ -1027,6 +1027,7 @@ void ssm_scan(const float* xbc, int ldx, const float* dt_raw, int lddt, const fl
     DLM_CHECK(N >= 1 && N <= 1024, "ssm_scan: state size 1..1024");
     {
         WalkParams w{};
+        w.longest = longest;
         w.q = xbc + (long long)heads * P + (long long)groups * N; w.ldq = ldx;
         w.k = xbc + (long long)heads * P; w.ldk = ldx;
         w.v = xbc; w.ldv = ldx;
@@ -1073,11 +1074,12 @@ void ssm_scan(const float* xbc, int ldx, const float* dt_raw, int lddt, const fl
 
 void delta_scan(const float* proj, int ld, int off_r, int off_k, int off_v, int off_a, const float* lw, int ldlw,
                 const float* a_bias, float* state, const int32_t* cu_q, const int32_t* state_slot, float* o, int R,
-                int heads, int d, float unit_eps, float decay_coef, cudaStream_t stream) {
+                int heads, int d, float unit_eps, float decay_coef, int longest, cudaStream_t stream) {
     if (R <= 0) return;
     DLM_CHECK(d >= 1 && d <= 512, "delta_scan: head size 1..512");
     {
         WalkParams w{};
+        w.longest = longest;
         w.q = proj + off_r; w.ldq = ld;
         w.k = proj + off_k; w.ldk = ld;
         w.v = proj + off_v; w.ldv = ld;

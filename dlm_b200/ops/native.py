@@ -33,6 +33,11 @@ class KernelError(RuntimeError):
     pass
 
 
+def _longest(batch, tokens: int) -> int:
+    """Tokens of the step's longest request (all the step's, where the batch does not say)."""
+    return int(getattr(batch, "max_q_len", 0)) or tokens
+
+
 class _Branch:
     """A piece of a step that may run beside the launching stream.  ``with branch:`` launches
     what is inside on a second stream that starts after everything launched so far;
@@ -250,7 +255,7 @@ class NativeOps:
         self.launches += 1
         self.k.ssm_scan(_p(xbc), xbc.stride(0), _p(dt_raw), 0 if dt_raw is None else dt_raw.stride(0), _p(dt_bias),
                         _p(A_log), _p(D), _p(state), _p(batch.cu_q), _p(batch.state_slot), _p(y), batch.num_requests,
-                        heads, P, N, groups, _p(fixed_decay), int(bool(silu_inputs)), self._stream())
+                        heads, P, N, groups, _p(fixed_decay), int(bool(silu_inputs)), _longest(batch, T), self._stream())
         return y
 
     def delta_scan(self, proj, offsets, lw, a_bias, state, batch, heads, d, unit_eps, decay_coef):
@@ -262,7 +267,7 @@ class NativeOps:
         self.launches += 1
         self.k.delta_scan(_p(proj), proj.stride(0), *[int(v) for v in offsets], _p(lw), lw.stride(0), _p(a_bias),
                           _p(state), _p(batch.cu_q), _p(batch.state_slot), _p(o), batch.num_requests, heads, d,
-                          float(unit_eps), float(decay_coef), self._stream())
+                          float(unit_eps), float(decay_coef), _longest(batch, T), self._stream())
         return o
 
     def selective_scan(self, x, dt_raw, bc, z, dt_bias, A_log, D, state, batch, out_dtype):
@@ -279,7 +284,7 @@ class NativeOps:
         self.launches += 1
         self.k.selective_scan(_p(x), x.stride(0), _p(dt_raw), dt_raw.stride(0), _p(bc), bc.stride(0), _p(z), z.stride(0),
                               _p(dt_bias), _p(A_log), _p(D), _p(state), _p(batch.cu_q), _p(batch.state_slot), _p(out),
-                              inner, batch.num_requests, inner, N, _dt(out_dtype), self._stream())
+                              inner, batch.num_requests, inner, N, _dt(out_dtype), _longest(batch, T), self._stream())
         return out
 
     def qk_norm_write(self, qkv, positions, qn_w, kn_w, eps, temp_coef, temp_every, slots, k_cache, v_cache, nh, nkv, d,
@@ -387,7 +392,7 @@ class NativeOps:
                           _p(beta), 0 if beta is None else beta.stride(0), _p(A_log), _p(decay_bias), _p(state),
                           _p(batch.cu_q), _p(batch.state_slot), _p(o), heads * dv, batch.num_requests, heads, qk_heads,
                           dk, dv, int(unit_eps is not None), float(unit_eps or 0.0), float(q_scale),
-                          0 if per_head else 1, float(tau or 0.0), self._stream())
+                          0 if per_head else 1, float(tau or 0.0), _longest(batch, T), self._stream())
         return o
 
     def head_norm_rope_write(self, qkv, positions, qn_w, kn_w, eps, inv_freq, rot_dims, interleaved, slots, k_cache,

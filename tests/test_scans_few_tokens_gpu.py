@@ -57,6 +57,60 @@ def test_a_state_may_lie_at_any_address(ops, N, P):
     ops.check_errors()
 
 
+def cut(T):
+    """``[(first, end), ...]``: steps of one, two, three, four, one, ... tokens, and one of six in the middle."""
+    out, at, n = [], 0, 0
+    while at < T:
+        step = min([1, 2, 3, 4, 1, 6][n % 6], T - at)
+        out.append((at, at + step))
+        at, n = at + step, n + 1
+    return out
+
+
+@pytest.mark.parametrize("N,P", SIZES)
+def test_few_tokens_give_the_same_bits(ops, N, P):
+    heads, lens, slots = 3, [21, 1, 18], [2, 0, 3]
+    starts = [0, 21, 22]
+    for name, run in scans(ops, N, P, sum(lens), heads).items():
+        first = randn(5, heads, N, P, seed=6, std=0.3)
+        whole_state, cut_state = first.clone(), first.clone()
+        whole = run(0, sum(lens), batch_of(lens, slots), whole_state)
+        for n, s, slot in zip(lens, starts, slots):
+            for a, e in cut(n):
+                got = run(s + a, s + e, batch_of([e - a], [slot]), cut_state)
+                assert torch.equal(got, whole[s + a:s + e]), (name, a, e)
+        assert torch.equal(cut_state, whole_state), name
+        # several short requests in one step
+        together, alone = first.clone(), first.clone()
+        both = run(0, 8, batch_of([3, 1, 4], [1, 4, 0]), together)
+        for a, e, slot in ((0, 3, 1), (3, 4, 4), (4, 8, 0)):
+            assert torch.equal(run(a, e, batch_of([e - a], [slot]), alone), both[a:e]), name
+        assert torch.equal(together, alone), name
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("inner,N", [(4, 1), (36, 8), (33, 9), (64, 16), (7, 33), (20, 256), (130, 12)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_selective_scan_of_few_tokens_gives_the_same_bits(ops, inner, N, dtype):
+    lens, slots, starts = [21, 1, 18], [2, 0, 3], [0, 21, 22]
+    T = sum(lens)
+    x, dt, z, bc = randn(T, inner, seed=1), randn(T, inner, seed=2), randn(T, inner, seed=3), randn(T, 2 * N, seed=4)
+    bias, A_log, D = randn(inner, seed=5), randn(inner, N, seed=6, std=0.5), randn(inner, seed=7)
+
+    def run(a, e, b, s):
+        return ops.selective_scan(x[a:e], dt[a:e], bc[a:e], z[a:e], bias, A_log, D, s, b, dtype)
+
+    first = randn(5, inner, N, seed=8, std=0.3)
+    whole_state, cut_state = first.clone(), first.clone()
+    whole = run(0, T, batch_of(lens, slots), whole_state)
+    for n, s, slot in zip(lens, starts, slots):
+        for a, e in cut(n):
+            got = run(s + a, s + e, batch_of([e - a], [slot]), cut_state)
+            assert torch.equal(got, whole[s + a:s + e]), (a, e)
+    assert torch.equal(cut_state, whole_state)
+    ops.check_errors()
+
+
 def test_removal_with_short_keys_and_no_floor(ops):
     """Keys of length 1e-20: their square is no normal number and its reciprocal out of range, their unit vector is fine."""
     heads, d, lens = 2, 16, [7, 1]
