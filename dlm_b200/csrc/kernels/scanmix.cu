@@ -65,7 +65,7 @@ __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-// 2^x on the special-function unit; what would be below 2^-126 is zero
+// 2^x on the special-function unit for x >= -126 (a result below that would become zero)
 __device__ __forceinline__ float ex2_ftz(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -73,14 +73,16 @@ __device__ __forceinline__ float ex2_ftz(float x) {
 }
 
 // One token of a channel: the lane's eight states move on; returns the sum of s C over the channel's states (in every lane).
-template <int PARTS>
+// TINY: a decay may lie below the smallest normal number; such tokens are rare, and ask the function that has such numbers.
+template <int PARTS, bool TINY>
 __device__ __forceinline__ float selective_token(f2 (&s)[4], const f2 (&a2)[4], const f2 (&bb)[4], const f2 (&cc)[4], float dt,
                                                  float xv) {
     const f2 dt2 = pack2(dt, dt), dx2 = pack2(dt * xv, dt * xv);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float2 w = unpack2(mul2(dt2, a2[i]));
-        s[i] = fma2(pack2(ex2_ftz(w.x), ex2_ftz(w.y)), s[i], mul2(dx2, bb[i]));
+        s[i] = fma2(TINY ? pack2(w.x < -126.f ? exp2f(w.x) : ex2_ftz(w.x), w.y < -126.f ? exp2f(w.y) : ex2_ftz(w.y))
+                         : pack2(ex2_ftz(w.x), ex2_ftz(w.y)), s[i], mul2(dx2, bb[i]));
     }
     f2 u = mul2(s[0], cc[0]), v = mul2(s[1], cc[1]);
     u = fma2(s[2], cc[2], u);
@@ -93,7 +95,7 @@ __device__ __forceinline__ float selective_token(f2 (&s)[4], const f2 (&a2)[4], 
 }
 
 // A prepared tile of n tokens: rows of rl floats [B | C | dt | x | gate], o the channel's output of the first.
-template <int PARTS, typename TOut>
+template <int PARTS, bool TINY, typename TOut>
 __device__ __forceinline__ void selective_tile(const float* buf, int n, int rl, int cp, int part, int col, bool live, f2 (&s)[4],
                                                const f2 (&a2)[4], float d_c, TOut* o, int ldo) {
     constexpr int NP = 8 * PARTS;
@@ -106,9 +108,16 @@ __device__ __forceinline__ void selective_tile(const float* buf, int n, int rl, 
         const ulonglong2 e1 = *reinterpret_cast<const ulonglong2*>(row + NP + 8 * part + 4);
         const float dt = row[2 * NP + col], xv = row[2 * NP + cp + col], gate = row[2 * NP + 2 * cp + col];
         const f2 bb[4] = {b0.x, b0.y, b1.x, b1.y}, cc[4] = {e0.x, e0.y, e1.x, e1.y};
-        const float sum = selective_token<PARTS>(s, a2, bb, cc, dt, xv);
+        const float sum = selective_token<PARTS, TINY>(s, a2, bb, cc, dt, xv);
         if (live && part == 0) o[(long long)tok * ldo] = from_f32<TOut>(fmaf(d_c, xv, sum) * gate);
     }
+}
+
+// (apart from the loop above, whose registers it would share)
+template <int PARTS, typename TOut>
+__device__ __noinline__ void selective_tile_tiny(const float* buf, int n, int rl, int cp, int part, int col, bool live, f2 (&s)[4],
+                                                 const f2 (&a2)[4], float d_c, TOut* o, int ldo) {
+    selective_tile<PARTS, true>(buf, n, rl, cp, part, col, live, s, a2, d_c, o, ldo);
 }
 
 struct SelectiveArgs {
@@ -122,10 +131,12 @@ struct SelectiveArgs {
     int ldo, inner, N, wide_bc;          // wide_bc: the eights of a token's B and C start on 16-byte boundaries
 };
 
-// The lane's eight states of channel c and their A log2 e (zeros beyond N, and in lanes without a channel).
+// The lane's eight states of channel c and their A log2 e (zeros beyond N, and in lanes without a channel); returns the least
+// of the latter.
 template <int PARTS>
-__device__ __forceinline__ void selective_load(const SelectiveArgs& p, const float* st, int c, int part, bool live, f2 (&s)[4],
-                                               f2 (&a2)[4]) {
+__device__ __forceinline__ float selective_load(const SelectiveArgs& p, const float* st, int c, int part, bool live, f2 (&s)[4],
+                                                f2 (&a2)[4]) {
+    float least = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         float sv[2], av[2];
@@ -138,7 +149,9 @@ __device__ __forceinline__ void selective_load(const SelectiveArgs& p, const flo
         }
         s[i] = pack2(sv[0], sv[1]);
         a2[i] = pack2(av[0], av[1]);
+        least = fminf(least, fminf(av[0], av[1]));
     }
+    return least;
 }
 __device__ __forceinline__ void selective_store(float* st, int N, int part, bool live, const f2 (&s)[4]) {
 #pragma unroll
@@ -189,7 +202,7 @@ __global__ void __launch_bounds__(32 * SCAN_WALKERS) selective_few_kernel(Select
             }
         }
         const float dt = softplus_f(p.dt_raw[t * p.lddt + ch] + bias), xv = p.x[t * p.ldx + ch], gate = silu_f(p.z[t * p.ldz + ch]);
-        const float sum = selective_token<PARTS>(s, a2, bb, cc, dt, xv);
+        const float sum = selective_token<PARTS, true>(s, a2, bb, cc, dt, xv);
         if (live && part == 0) out[t * p.ldo + c] = from_f32<TOut>(fmaf(d_c, xv, sum) * gate);
     }
     selective_store(st, N, part, live, s);
@@ -203,12 +216,16 @@ selective_scan_kernel(SelectiveArgs p, TOut* out, int walkers, int tile_tokens, 
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     constexpr int NP = 8 * PARTS, CW = 32 / PARTS;        // states as stored; channels of a warp
     extern __shared__ __align__(16) float sm[];           // [STAGES][tile][B: NP | C: NP | dt | x | gate: cp each]
+    __shared__ float s_least[SCAN_WALKERS * 32];          // a channel's most negative A log2 e
+    __shared__ int s_tiny[SCAN_STAGES];                   // a decay of the tile may lie below the smallest normal number
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int chans = walkers * CW, cp = (chans + 3) & ~3, rl = 2 * NP + 3 * cp;
     const int c0 = blockIdx.x * chans, nch = min(chans, inner - c0);
     const int r = blockIdx.y;
     const int t0 = p.cu_q[r], t1 = p.cu_q[r + 1];
     const int n_tiles = (t1 - t0 + tile_tokens - 1) / tile_tokens;
+
+    if (threadIdx.x < SCAN_STAGES) s_tiny[threadIdx.x] = 0;
 
     if (warp >= walkers) {
         const int helper = warp - walkers;
@@ -252,17 +269,22 @@ selective_scan_kernel(SelectiveArgs p, TOut* out, int walkers, int tile_tokens, 
             float* buf = sm + (size_t)(k % SCAN_STAGES) * tile_tokens * rl;
             const int n = min(tile_tokens, t1 - (t0 + k * tile_tokens));
             __syncwarp();                 // every lane has waited for its own copies
+            bool tiny = false;
             for (int tok = helper; tok < n; tok += SCAN_HELPERS) {
                 float* dt = buf + (size_t)tok * rl + 2 * NP;
                 float* gate = dt + 2 * cp;
                 for (int i = lane; i < nch; i += 32) {
-                    dt[i] = softplus_f(dt[i] + p.dt_bias[c0 + i]);
+                    const float step = softplus_f(dt[i] + p.dt_bias[c0 + i]);
+                    dt[i] = step;
+                    tiny = tiny || step * s_least[i] < -126.f;
                     gate[i] = silu_f(gate[i]);
                 }
             }
+            if (tiny) s_tiny[k % SCAN_STAGES] = 1;
         };
         for (int k = 0; k < SCAN_STAGES - 1; ++k) fetch(k);
         copies_wait<SCAN_STAGES - 2>();
+        __syncthreads();                  // the channels' decays are known
         if (n_tiles > 0) prepare(0);
         __syncthreads();
         for (int k = 0; k < n_tiles; ++k) {              // the walkers are at tile k
@@ -279,15 +301,28 @@ selective_scan_kernel(SelectiveArgs p, TOut* out, int walkers, int tile_tokens, 
     const bool live = c < inner;
     float* st = p.state + ((long long)p.state_slot[r] * inner + (live ? c : 0)) * N;
     f2 s[4], a2[4];
-    selective_load<PARTS>(p, st, c, part, live, s, a2);
+    float least = selective_load<PARTS>(p, st, c, part, live, s, a2);
+#pragma unroll
+    for (int o = 1; o < PARTS; o <<= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+    if (part == 0) s_least[col] = least;
     const float d_c = live ? p.D[c] : 0.f;
     __syncthreads();
+    __syncthreads();                      // tile 0 is prepared
     for (int k = 0; k < n_tiles; ++k) {
         const float* buf = sm + (size_t)(k % SCAN_STAGES) * tile_tokens * rl;
         const int first = t0 + k * tile_tokens, n = min(tile_tokens, t1 - first);
         TOut* o = out + (long long)first * p.ldo + c;
-        selective_tile<PARTS>(buf, n, rl, cp, part, col, live, s, a2, d_c, o, p.ldo);
+        if (s_tiny[k % SCAN_STAGES] != 0) {
+            f2 kept[4] = {s[0], s[1], s[2], s[3]};
+            selective_tile_tiny<PARTS, TOut>(buf, n, rl, cp, part, col, live, kept, a2, d_c, o, p.ldo);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[i] = kept[i];
+        } else {
+            selective_tile<PARTS, false>(buf, n, rl, cp, part, col, live, s, a2, d_c, o, p.ldo);
+        }
         __syncthreads();
+        // (nobody reads this tile's any more; it is set again for tile k + 4, after two more barriers)
+        if (threadIdx.x == 0) s_tiny[k % SCAN_STAGES] = 0;
     }
     selective_store(st, N, part, live, s);
 }

@@ -111,6 +111,25 @@ def test_selective_scan_of_few_tokens_gives_the_same_bits(ops, inner, N, dtype):
     ops.check_errors()
 
 
+def test_selective_scan_keeps_decays_below_the_normal_numbers(ops):
+    """Decays of 2^-127 to 2^-140 on a state of 2^120 and more: what is left of it is a normal number."""
+    inner, N = 32, 16
+    powers = torch.linspace(-140, -100, inner * N, dtype=torch.float64).view(inner, N)
+    A_log = torch.log(-powers * 0.6931471805599453).float().to(DEV)      # decay 2^power at a step size of one
+    bias = torch.full((inner,), 0.5413248546 - 1.0, device=DEV)         # softplus(ln(e - 1)) = 1
+    for tokens in (1, 6):                                               # the kernel without a ring and the one with it
+        dt = torch.full((tokens, inner), -60.0, device=DEV)             # the tokens after the first leave the state as it is
+        dt[0] = 1.0
+        zero, none = torch.zeros(tokens, inner, device=DEV), torch.zeros(inner, device=DEV)
+        s = torch.full((1, inner, N), 2.0 ** 120, device=DEV)
+        ops.selective_scan(zero, dt, torch.zeros(tokens, 2 * N, device=DEV), zero, bias, A_log, none, s, batch_of([tokens], [0]),
+                           torch.float32)
+        step = torch.nn.functional.softplus((dt[0] + bias).double().cpu())[:, None]
+        want = 2.0 ** 120 * torch.exp(-step * torch.exp(A_log.double().cpu()))
+        # an argument of 140 carries 2^-24 of itself, some 1e-5 of the decay; a decay of 2^-140 keeps nine bits
+        assert torch.allclose(s[0].double().cpu(), want, rtol=4e-3)
+
+
 def test_removal_with_short_keys_and_no_floor(ops):
     """Keys of length 1e-20: their square is no normal number and its reciprocal out of range, their unit vector is fine."""
     heads, d, lens = 2, 16, [7, 1]
