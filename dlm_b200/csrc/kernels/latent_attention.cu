@@ -542,6 +542,61 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
     }
 }
 
+// The rows of a run once more, a warp a row and straight from the cache: a row's sum runs over the keys its token sees alone.  For
+// runs with a sum that is not finite, which a latent may have caused that the token does not see.
+template <int HG>
+__device__ __noinline__ void latent_rows_one_by_one(const __nv_bfloat16* s_q, int qp, const __nv_bfloat16* cache,
+                                                    const int32_t* table, int table_width, const float* sink,
+                                                    __nv_bfloat16* lat, int t0, int n_tok, int p_first, int h0, int Tn, int H,
+                                                    int rank, int width, int page_size, int total_pages, int window,
+                                                    float scale) {
+    const int lane = threadIdx.x & 31;
+    for (int row = threadIdx.x >> 5; row < n_tok * HG; row += (int)(blockDim.x >> 5)) {
+        const int i = row / HG, h = h0 + row % HG, p = p_first + i;
+        if (h >= H) continue;
+        const int lo = window > 0 ? max(p - window + 1, 0) : 0;
+        float m = -INFINITY, l = 0.f, acc[16];               // entries lane, lane + 32, ... (the latent has at most 512)
+#pragma unroll
+        for (int u = 0; u < 16; ++u) acc[u] = 0.f;
+        for (int j0 = lo / LA_KC * LA_KC; j0 <= p; j0 += LA_KC) {
+            const int j = j0 + lane;
+            long long off = -1;
+            if (j >= lo && j <= p) {
+                const int lp = j / page_size, page = lp < table_width ? table[lp] : -1;
+                if (page >= 0 && page < total_pages) off = ((long long)page * page_size + (j - lp * page_size)) * width;
+            }
+            float sc = 0.f;
+            if (off >= 0)
+                for (int c = 0; c < width; ++c)
+                    sc = fmaf(__bfloat162float(s_q[(size_t)row * qp + c]), __bfloat162float(cache[off + c]), sc);
+            sc = j >= lo && j <= p ? sc * scale : -INFINITY;
+            const float m_new = fmaxf(m, warp_max(sc));
+            const float w = m_new > -INFINITY ? expf(sc - m_new) : 0.f, corr = m_new > -INFINITY ? expf(m - m_new) : 1.f;
+            l = l * corr + warp_sum(w);
+            m = m_new;
+#pragma unroll
+            for (int u = 0; u < 16; ++u) acc[u] *= corr;
+            for (int kk = 0; kk < LA_KC; ++kk) {
+                const float wk = __shfl_sync(0xffffffffu, w, kk);
+                const long long ok = __shfl_sync(0xffffffffu, off, kk);
+                if (ok < 0) continue;
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    if (lane + 32 * u < rank) acc[u] = fmaf(wk, __bfloat162float(cache[ok + lane + 32 * u]), acc[u]);
+            }
+        }
+        const float snk = sink ? sink[h] : -INFINITY;
+        const float mm = fmaxf(m, snk);
+        const float f = l > 0.f ? expf(m - mm) : 0.f;
+        const float den = l * f + (sink ? expf(snk - mm) : 0.f);
+        const float w = den > 0.f ? f / den : 0.f;
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (lane + 32 * u < rank)
+                lat[((long long)h * Tn + t0 + i) * rank + lane + 32 * u] = __float2bfloat16_rn(acc[u] * w);
+    }
+}
+
 // The same for the tokens of a prompt: one block a run of 64 / HG tokens of a request and HG (8 or 16) of their heads, 64
 // rows of queries that meet every staged key row.  A token's own block (above) fetches its whole window for 16 rows, so
 // the fetch and the shared-memory reads of the keys bound it; here they are spent on four times the rows.  Per chunk of 32 keys:
@@ -775,6 +830,19 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
                 }
             }
         }
+    }
+    // A key's weight is zero for a token of the run that does not see it, but zero times an infinity is not
+    bool bad = false;
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) bad = bad || !isfinite(acc[m][n][e]);
+    if (__syncthreads_or(bad)) {
+        latent_rows_one_by_one<HG>(s_q, qp, cache, table, table_width, sink, lat, t0, n_tok, p_first, h0, Tn, H, rank, width,
+                                   page_size, total_pages, window, scale);
+        return;
     }
     if (sub == 0) {
         s_m[srow] = m_run;
