@@ -877,21 +877,29 @@ __global__ void latent_merge_kernel(const float* partial, int n_splits, const fl
     dep_launch_next();
     const int t = blockIdx.x, h = blockIdx.y;
     const float* base = partial + ((long long)t * H + h) * n_splits * (rank + 2);
+    __shared__ float s_max[32], s_sum[32];                   // of the splits (at most 32); then s_max: their weights, -1: nothing seen
     const float snk = sink ? sink[h] : -INFINITY;
-    float mm = snk;
-    for (int s = 0; s < n_splits; ++s) mm = fmaxf(mm, base[(long long)s * (rank + 2)]);
-    float den = sink ? expf(snk - mm) : 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float* ps = base + (long long)s * (rank + 2);
-        if (ps[1] > 0.f) den += ps[1] * expf(ps[0] - mm);
+    if (threadIdx.x < n_splits) {
+        s_max[threadIdx.x] = base[(long long)threadIdx.x * (rank + 2)];
+        s_sum[threadIdx.x] = base[(long long)threadIdx.x * (rank + 2) + 1];
     }
+    __syncthreads();
+    float mm = snk;
+    for (int s = 0; s < n_splits; ++s) mm = fmaxf(mm, s_max[s]);
+    __syncthreads();
+    if (threadIdx.x < n_splits) s_max[threadIdx.x] = s_sum[threadIdx.x] > 0.f ? expf(s_max[threadIdx.x] - mm) : -1.f;
+    __syncthreads();
+    float den = sink ? expf(snk - mm) : 0.f;
+    for (int s = 0; s < n_splits; ++s)
+        if (s_max[s] >= 0.f) den += s_sum[s] * s_max[s];
     const float inv = den > 0.f ? 1.0f / den : 0.f;
     T* dst = lat + ((long long)h * Tn + t) * rank;
     for (int r = threadIdx.x; r < rank; r += blockDim.x) {
         float v = 0.f;
+#pragma unroll 4
         for (int s = 0; s < n_splits; ++s) {
-            const float* ps = base + (long long)s * (rank + 2);
-            if (ps[1] > 0.f) v = fmaf(ps[2 + r], expf(ps[0] - mm), v);
+            const float x = base[(long long)s * (rank + 2) + 2 + r], w = s_max[s];
+            if (w >= 0.f) v = fmaf(x, w, v);
         }
         dst[r] = from_f32<T>(v * inv);
     }
