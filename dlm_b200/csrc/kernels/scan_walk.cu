@@ -18,7 +18,7 @@
 //
 // Measured, one request of 2,048 tokens, before (a lane one column, 4-16 rows, everything done by all warps) and now: state space, 64
 // heads of 128 x 64: 824 -> 286 us; retention, 16 heads of 64 x 128: 534 -> 158; gated linear attention, 16 heads of 64 x 128:
-// 577 -> 198; gated delta rule, 16 heads of 128 x 128: 754 -> 352; removal form, 32 heads of 64 x 64: 1,225 -> 305.
+// 577 -> 198; gated delta rule, 16 heads of 128 x 128: 754 -> 352; removal form, 32 heads of 64 x 64: 1,225 -> 319.
 #include "api.h"
 #include "common.cuh"
 #include "scan_walk.h"
@@ -187,10 +187,12 @@ __device__ __forceinline__ void walk_token(f2 (&s)[4][CPL], const f2 (&q)[4], co
                 for (int i = 0; i < 4; ++i) s[i][c] = fma2(k[i], uu, s[i][c]);
                 with[c] = u;
             } else {
-                const f2 kk = pack2(ks[c], ks[c]), vv = pack2(v[c], v[c]);
+                // (what is removed first, then k v^T: the other way round rounds the larger sum)
+                const float us = ks[c] * sc.x;
+                const f2 uu = pack2(us, us), vv = pack2(v[c], v[c]);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s[i][c] = fma2(rr[i], kk, fma2(k[i], vv, mul2(a[i], s[i][c])));
-                with[c] = fmaf(v[c], sc.z, -(sc.y * ks[c]));
+                for (int i = 0; i < 4; ++i) s[i][c] = fma2(k[i], vv, fma2(rr[i], uu, mul2(a[i], s[i][c])));
+                with[c] = fmaf(v[c], sc.z, -(sc.y * us));
             }
         }
     }
@@ -341,10 +343,11 @@ __global__ void __launch_bounds__(32 * MOST_WALKERS, 3) scan_few_kernel(WalkPara
             for (int i = 0; i < 8; ++i) rr[i] *= k[i];
             const float kk = dot(k, k), qk = dot(q, k), qr = dot(q, rr);
             const float inv = 1.0f / sqrtf(kk + p.unit_eps);
-            sc.y = qr * inv * inv;
+            sc.x = inv;
+            sc.y = qr * inv;
             sc.z = qk;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { q[i] *= a[i]; rr[i] = -rr[i] * inv * inv; }
+            for (int i = 0; i < 8; ++i) { q[i] *= a[i]; rr[i] = -rr[i] * inv; }
         }
         f2 q2[4], k2[4], a2[4], r2[4];
 #pragma unroll
@@ -510,13 +513,14 @@ __global__ void __launch_bounds__(32 * MOST_WARPS, 1) scan_walk_kernel(WalkParam
                             }
                         }
                     } else {
-                        // k stays as it is (it carries v); the removal's r u u^T S = (r k / |k| / |k|)(k^T S): divided twice, so
+                        // k stays as it is (it carries v); the removal's r u u^T S = (r k / |k|)(k^T S / |k|): divided twice, so
                         // that nothing leaves the 32-bit range that u and r u do not leave; q meets the old state through
                         // the decays
                         qr = token_sum(qr);
                         const float inv = 1.0f / sqrtf(kk + p.unit_eps);
                         if (mine) {
-                            if (lt == 0) row[off_s + 1] = qr * inv * inv;
+                            if (lt == 0) row[off_s] = inv;
+                            if (lt == 0) row[off_s + 1] = qr * inv;
                             if (lt == 1) row[off_s + 2] = qk;
 #pragma unroll
                             for (int q = 0; q < QL; ++q) {
@@ -524,8 +528,8 @@ __global__ void __launch_bounds__(32 * MOST_WARPS, 1) scan_walk_kernel(WalkParam
                                 *reinterpret_cast<float4*>(row + i) = make_float4(qv[4 * q] * av[4 * q], qv[4 * q + 1] * av[4 * q + 1],
                                                                                   qv[4 * q + 2] * av[4 * q + 2], qv[4 * q + 3] * av[4 * q + 3]);
                                 *reinterpret_cast<float4*>(row + 2 * NP + i) = make_float4(av[4 * q], av[4 * q + 1], av[4 * q + 2], av[4 * q + 3]);
-                                *reinterpret_cast<float4*>(row + 3 * NP + i) = make_float4(-rv[4 * q] * inv * inv, -rv[4 * q + 1] * inv * inv,
-                                                                                           -rv[4 * q + 2] * inv * inv, -rv[4 * q + 3] * inv * inv);
+                                *reinterpret_cast<float4*>(row + 3 * NP + i) = make_float4(-rv[4 * q] * inv, -rv[4 * q + 1] * inv,
+                                                                                           -rv[4 * q + 2] * inv, -rv[4 * q + 3] * inv);
                             }
                         }
                     }
