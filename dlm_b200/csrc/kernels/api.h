@@ -271,20 +271,23 @@ void latent_q_split(const float* q, int ldq, const int32_t* positions, const flo
 // sink f32 [H] or nullptr (a logit per head that joins the softmax's maximum and denominator only); cache
 // [pages, 1, page_size, rank + dr] and lat[H, T, rank] (the normalised weighted sums of latent rows) in `dtype`.
 // A query at position p sees keys j with 0 <= p - j < window (window 0: all).  cu_q [R + 1]: where each of the step's R
-// requests' tokens (at consecutive positions) begin.  n_splits (from
-// latent_attention_splits) > 1 cuts every token's keys over that many blocks; `partial` then holds
-// T * H * n_splits * (rank + 2) floats of scratch and a second kernel merges.  fast != 0 allows the tensor-core
+// requests' tokens (at consecutive positions) begin; the `apart` of them that bring one token (all that do, or 0) go to a kernel
+// of their own.  Returns the number of launches.  n_splits and apart come from latent_attention_plan: n_splits > 1 cuts every
+// token's keys (every such request's, where they go apart) over that many blocks; `partial` then holds the plan's floats of
+// scratch and another kernel merges.  fast != 0 allows the tensor-core
 // kernel (bfloat16, rank a multiple of 128 up to 512, dr a multiple of 8).
-void latent_attention(const float* q_lat, const float* q_rot, const float* sink, const void* cache,
+int latent_attention(const float* q_lat, const float* q_rot, const float* sink, const void* cache,
                       const int32_t* block_table, int table_width, const int32_t* token_req, const int32_t* positions,
-                      const int32_t* cu_q, int R, void* lat, float* partial, int n_splits, int T, int H, int dr, int rank,
+                      const int32_t* cu_q, int R, int apart, void* lat, float* partial, int n_splits, int T, int H, int dr, int rank,
                       int page_size, int total_pages, int window, float scale, int dtype, int fast, cudaStream_t stream);
 // out[t, h * dv + d] = val[h * T + t, d] * sigmoid(gate[t, h]) in `dtype` (val f32 [H, T, dv]; gate f32 raw, or nullptr)
 void latent_gate_out(const float* val, const float* gate, int ldg, void* out, int T, int H, int dv, int dtype,
                      cudaStream_t stream);
-// Splits that fill the machine for a step of T tokens of R requests whose longest visible range is max_keys (1 in 32-bit, where
-// the order of every sum is fixed).
-int latent_attention_splits(int T, int R, int H, int rank, int dr, int max_keys, int dtype, int fast);
+// How a step of T tokens of R requests, `singles` of which bring one token, is run when its longest visible range is max_keys:
+// splits that fill the machine (1 in 32-bit, where the order of every sum is fixed), floats of scratch, and whether the requests
+// of one token go apart from the prompts (how many of them do).
+struct LatentPlan { int n_splits, apart; long long scratch; };
+LatentPlan latent_attention_plan(int T, int R, int singles, int H, int rank, int dr, int max_keys, int dtype, int fast);
 
 // ---- gated recurrences with a matrix state, per-head norms, sublayers with a norm on both sides (gatedmix.cu) ----
 

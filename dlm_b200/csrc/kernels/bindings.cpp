@@ -209,16 +209,19 @@ PYBIND11_MODULE(_dlm_kernels, m) {
                               st(stream));
     });
     m.def("latent_attention", [](u64 q_lat, u64 q_rot, u64 sink, u64 cache, u64 block_table, int table_width,
-                                 u64 token_req, u64 positions, u64 cu_q, int R, u64 lat, u64 partial, int n_splits, int T, int H, int dr,
+                                 u64 token_req, u64 positions, u64 cu_q, int R, int apart, u64 lat, u64 partial, int n_splits, int T, int H, int dr,
                                  int rank, int page_size, int total_pages, int window, float scale, int dtype, int fast,
                                  u64 stream) {
-        dlmk::latent_attention(ptr<const float>(q_lat), ptr<const float>(q_rot), ptr<const float>(sink),
+        return dlmk::latent_attention(ptr<const float>(q_lat), ptr<const float>(q_rot), ptr<const float>(sink),
                                ptr<const void>(cache), ptr<const int32_t>(block_table), table_width,
-                               ptr<const int32_t>(token_req), ptr<const int32_t>(positions), ptr<const int32_t>(cu_q), R, ptr<void>(lat),
+                               ptr<const int32_t>(token_req), ptr<const int32_t>(positions), ptr<const int32_t>(cu_q), R, apart, ptr<void>(lat),
                                ptr<float>(partial), n_splits, T, H, dr, rank, page_size, total_pages, window, scale, dtype,
                                fast, st(stream));
     });
-    m.def("latent_attention_splits", &dlmk::latent_attention_splits);
+    m.def("latent_attention_plan", [](int T, int R, int singles, int H, int rank, int dr, int max_keys, int dtype, int fast) {
+        const dlmk::LatentPlan p = dlmk::latent_attention_plan(T, R, singles, H, rank, dr, max_keys, dtype, fast);
+        return py::make_tuple(p.n_splits, p.apart, p.scratch);
+    });
     m.def("gated_scan", [](u64 q, int ldq, u64 k, int ldk, u64 v, int ldv, u64 dec, int ldd, u64 beta, int ldb, u64 A_log,
                            u64 dec_bias, u64 state, u64 cu_q, u64 state_slot, u64 o, int ldo, int R, int heads,
                            int qk_heads, int dk, int dv, int unit, float unit_eps, float q_scale, int decay_kind,

@@ -343,12 +343,28 @@ latent_attention_kernel(const float* __restrict__ q_lat, const float* __restrict
 constexpr int LM_ROWS = 16;
 constexpr int LM_PP = LA_KC + 8;           // row pitch of the weights (bfloat16)
 
+// The token of the step's n-th request that brings one token (cu_q as in the step); -1: there is none.  Asked by a whole warp.
+__device__ __forceinline__ int nth_single(const int32_t* cu_q, int R, int n) {
+    const int lane = threadIdx.x & 31;
+    for (int base = 0; base < R; base += 32) {
+        const int r = base + lane, at = r < R ? cu_q[r] : 0;
+        unsigned mask = __ballot_sync(0xffffffffu, r < R && cu_q[r + 1] - at == 1);
+        if (n < __popc(mask)) {
+            for (; n > 0; --n) mask &= mask - 1;
+            return __shfl_sync(0xffffffffu, at, __ffs(mask) - 1);
+        }
+        n -= __popc(mask);
+    }
+    return -1;
+}
+
 template <int NT>
 __global__ void __launch_bounds__(LA_THREADS)
 latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_rot,
                             const float* __restrict__ sink, const __nv_bfloat16* __restrict__ cache,
                             const int32_t* __restrict__ block_table, int table_width,
                             const int32_t* __restrict__ token_req, const int32_t* __restrict__ positions,
+                            const int32_t* __restrict__ singles, int R,
                             __nv_bfloat16* lat, float* partial, int Tn, int H, int dr, int rank, int page_size,
                             int total_pages, int window, float scale, int n_splits, int* err) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
@@ -366,7 +382,9 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
     float* s_m = s_s + 2 * LM_ROWS * LA_KC;                 // [16]
     float* s_l = s_m + LM_ROWS;
     float* s_corr = s_l + LM_ROWS;
-    const int t = blockIdx.x;
+    const int t = singles != nullptr ? nth_single(singles, R, blockIdx.x) : (int)blockIdx.x;
+    if (t < 0) return;
+    const int req = token_req[t];
     const int h0 = blockIdx.y * LM_ROWS;
     const int hg = min(LM_ROWS, H - h0);
     const int ks_id = blockIdx.z;
@@ -394,7 +412,6 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
 #pragma unroll
     for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
 
-    const int req = token_req[t];
     const int32_t* table = block_table + (long long)req * table_width;
     const int lo = window > 0 ? max(p - window + 1, 0) : 0;
     const int c_first = lo / LA_KC, c_last = p / LA_KC;
@@ -517,7 +534,7 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
         const int row = g + 8 * rr;
         if (row >= hg) continue;
         if (n_splits > 1) {
-            float* dst = partial + (((long long)t * H + h0 + row) * n_splits + ks_id) * (rank + 2);
+            float* dst = partial + (((long long)blockIdx.x * H + h0 + row) * n_splits + ks_id) * (rank + 2);
             if (warp == 0 && tq == 0) {
                 dst[0] = s_m[row];
                 dst[1] = s_l[row];
@@ -613,7 +630,7 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
                              const float* __restrict__ sink, const __nv_bfloat16* __restrict__ cache,
                              const int32_t* __restrict__ block_table, int table_width, const int32_t* __restrict__ cu_q, int R,
                              const int32_t* __restrict__ positions, __nv_bfloat16* lat, int Tn, int H, int dr, int rank,
-                             int page_size, int total_pages, int window, float scale, int* err) {
+                             int page_size, int total_pages, int window, float scale, int skip_single, int* err) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     typedef __nv_bfloat16 bf16;
     constexpr int TB = LR_ROWS / HG, THREADS = 32 * W, KQ = W / 4, TPR = W / 2, KPT = LA_KC / TPR;
@@ -637,7 +654,7 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
         int acc = 0;
         s_map[0] = -1;
         for (int r = 0; r < R; ++r) {
-            const int b = cu_q[r], e = cu_q[r + 1], runs = (e - b + TB - 1) / TB;
+            const int b = cu_q[r], e = cu_q[r + 1], runs = skip_single && e - b == 1 ? 0 : (e - b + TB - 1) / TB;
             if (want < acc + runs) {
                 s_map[0] = r;
                 s_map[1] = b + (want - acc) * TB;
@@ -666,14 +683,14 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
         const int row = idx / (qp - width), c = idx - row * (qp - width);
         s_keys0[(size_t)row * qp + width + c] = __float2bfloat16_rn(0.f);
     }
+    const int32_t* table = block_table + (long long)req * table_width;
+    const int p_first = positions[t0], p_last = positions[t0 + n_tok - 1];
     float acc[4][NT][4];
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f;
 
-    const int32_t* table = block_table + (long long)req * table_width;
-    const int p_first = positions[t0], p_last = positions[t0 + n_tok - 1];
     const int lo = window > 0 ? max(p_first - window + 1, 0) : 0;
     const int c_begin = lo / LA_KC, c_end = p_last / LA_KC + 1;
     auto stage = [&](int ch, int which) {
@@ -872,11 +889,12 @@ latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __res
 // Merges the splits of a (token, head) in order and normalises as above.  One block a (token, head).
 template <typename T>
 __global__ void latent_merge_kernel(const float* partial, int n_splits, const float* __restrict__ sink,
-                                    T* lat, int Tn, int H, int rank) {
+                                    const int32_t* __restrict__ cu_q, int R, T* lat, int Tn, int H, int rank) {
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
-    const int t = blockIdx.x, h = blockIdx.y;
-    const float* base = partial + ((long long)t * H + h) * n_splits * (rank + 2);
+    const int t = cu_q != nullptr ? nth_single(cu_q, R, blockIdx.x) : (int)blockIdx.x, h = blockIdx.y;
+    if (t < 0) return;
+    const float* base = partial + ((long long)blockIdx.x * H + h) * n_splits * (rank + 2);
     __shared__ float s_max[32], s_sum[32];                   // of the splits (at most 32); then s_max: their weights, -1: nothing seen
     const float snk = sink ? sink[h] : -INFINITY;
     if (threadIdx.x < n_splits) {
@@ -953,7 +971,7 @@ void launch_latent(const float* q_lat, const float* q_rot, const float* sink, co
         error_flag_ptr());
     check_launch("latent_attention");
     if (n_splits > 1) {
-        launch_dep(latent_merge_kernel<T>, dim3(Tn, H), dim3(128), 0, stream, partial, n_splits, sink, static_cast<T*>(lat), Tn, H, rank);
+        launch_dep(latent_merge_kernel<T>, dim3(Tn, H), dim3(128), 0, stream, partial, n_splits, sink, nullptr, 0, static_cast<T*>(lat), Tn, H, rank);
         check_launch("latent_merge");
     }
 }
@@ -978,8 +996,10 @@ size_t rows_smem(int rank, int dr) {
     return ((size_t)(LR_ROWS + 2 * LA_KC) * qp + 2 * LR_ROWS * LM_PP) * sizeof(__nv_bfloat16) +
            (rows_warps(rank) / 4 * LR_ROWS * LR_SP + 3 * LR_ROWS) * sizeof(float);
 }
-// The many-row kernel: prompts (eight tokens a request and more) that give it a block for every other multiprocessor, and rows
-// of which 128 fit in shared memory.
+// The many-row kernel: prompts (eight tokens a request and more: a run of few tokens leaves its rows empty; 64 requests of 8
+// tokens and 16 heads of 512 + 64: 23 us against 35 of the kernel a token, with 4 such heads of 128 they do not reach the line below)
+// that give it a block for every other multiprocessor (300 tokens of 16 heads: 58 us against 61, with a rank of 384 56 against
+// 54; 1,024 tokens: 158 against 310), and rows of which 128 fit in shared memory.
 bool latent_use_rows(int T, int R, int H, int rank, int dr, int dtype, int fast) {
     const int hg = rows_heads(H);
     return latent_use_mma(dtype, rank, dr, fast) && R > 0 && T >= 8 * R && rows_smem(rank, dr) <= 226 * 1024 &&
@@ -987,17 +1007,28 @@ bool latent_use_rows(int T, int R, int H, int rank, int dr, int dtype, int fast)
 }
 }  // namespace
 
-int latent_attention_splits(int T, int R, int H, int rank, int dr, int max_keys, int dtype, int fast) {
-    if (dtype == F32 || T <= 0) return 1;       // 32-bit: one order of summation whatever the step holds
-    if (latent_use_rows(T, R, H, rank, dr, dtype, fast)) return 1;
+// Requests of one token beside prompts go apart where their keys may be many: a run of one token walks them with one row in four or
+// eight filled, behind the barriers of 64 rows (63 such requests with 4,000 keys beside 961 tokens, 16 heads of 512 + 64: 723 us
+// together, 361 apart, 457 with a block a token for all; 15 of them beside 1,024 tokens: 724, 226 and 458).  With up to 1,024 keys
+// the walk ends before the prompts' does (the latter step with 1,000 keys: 294 us together against 318 with a block a token).
+LatentPlan latent_attention_plan(int T, int R, int singles, int H, int rank, int dr, int max_keys, int dtype, int fast) {
+    LatentPlan plan{1, 0, 0};                   // (no splits, nothing apart, no scratch)
+    if (dtype == F32 || T <= 0) return plan;    // 32-bit: one order of summation whatever the step holds
+    if (singles > 0 && max_keys > 1024 && latent_use_rows(T - singles, R - singles, H, rank, dr, dtype, fast)) plan.apart = singles;
+    else if (latent_use_rows(T, R, H, rank, dr, dtype, fast)) return plan;
+    const int tokens = plan.apart > 0 ? plan.apart : T;
     const int blocks = latent_use_mma(dtype, rank, dr, fast)
-                           ? T * ((H + LM_ROWS - 1) / LM_ROWS)
-                           : T * ((H + heads_per_block(H) - 1) / heads_per_block(H));
+                           ? tokens * ((H + LM_ROWS - 1) / LM_ROWS)
+                           : tokens * ((H + heads_per_block(H) - 1) / heads_per_block(H));
     int want = (2 * sm_count() + blocks - 1) / blocks;
     const int chunks = (max_keys < 1 ? 1 : max_keys) / LA_KC + 1;
     if (want > chunks) want = chunks;
     if (want > 32) want = 32;
-    return want < 1 ? 1 : want;
+    if (want > 1) {
+        plan.n_splits = want;
+        plan.scratch = (long long)tokens * H * want * (rank + 2);
+    }
+    return plan;
 }
 
 void latent_q_split(const float* q, int ldq, const int32_t* positions, const float* inv_freq, int rot_dims,
@@ -1024,14 +1055,17 @@ void latent_gate_out(const float* val, const float* gate, int ldg, void* out, in
     check_launch("latent_gate_out");
 }
 
-void latent_attention(const float* q_lat, const float* q_rot, const float* sink, const void* cache,
+int latent_attention(const float* q_lat, const float* q_rot, const float* sink, const void* cache,
                       const int32_t* block_table, int table_width, const int32_t* token_req, const int32_t* positions,
-                      const int32_t* cu_q, int R, void* lat, float* partial, int n_splits, int T, int H, int dr, int rank,
+                      const int32_t* cu_q, int R, int apart, void* lat, float* partial, int n_splits, int T, int H, int dr, int rank,
                       int page_size, int total_pages, int window, float scale, int dtype, int fast, cudaStream_t stream) {
-    if (T <= 0) return;
+    if (T <= 0) return 0;
     DLM_CHECK(rank >= 1 && rank <= 1024, "latent_attention: latent size 1..1024");
     DLM_CHECK(n_splits >= 1 && (n_splits == 1 || partial != nullptr), "latent_attention: splits need a scratch buffer");
-    if (n_splits == 1 && latent_use_rows(T, R, H, rank, dr, dtype, fast)) {
+    DLM_CHECK(apart >= 0 && apart <= R, "latent_attention: requests of one token are some of the requests");
+    const bool rows = (apart > 0 || n_splits == 1) && latent_use_rows(T - apart, R - apart, H, rank, dr, dtype, fast);
+    DLM_CHECK(rows || apart == 0, "latent_attention: requests are taken apart from prompts only");
+    if (rows) {
         const int hg = rows_heads(H), tb = LR_ROWS / hg;
         const size_t smem = rows_smem(rank, dr);
         const dim3 grid(T / tb + R, (H + hg - 1) / hg);     // every request may end in a partial run
@@ -1042,7 +1076,7 @@ void latent_attention(const float* q_lat, const float* q_rot, const float* sink,
         kern<<<grid, 32 * W, smem, stream>>>(q_lat, q_rot, sink, static_cast<const __nv_bfloat16*>(cache),            \
                                              block_table, table_width, cu_q, R, positions,                            \
                                              static_cast<__nv_bfloat16*>(lat), T, H, dr, rank, page_size,             \
-                                             total_pages, window, scale, error_flag_ptr());                           \
+                                             total_pages, window, scale, apart > 0 ? 1 : 0, error_flag_ptr());        \
     } while (0)
 #define DLM_LROWS_H(NT, W) do { if (hg == 8) DLM_LROWS(NT, 8, W); else DLM_LROWS(NT, 16, W); } while (0)
         switch (rank / 64) {                                // NT = rank / (8 W), W = rows_warps(rank)
@@ -1054,19 +1088,20 @@ void latent_attention(const float* q_lat, const float* q_rot, const float* sink,
 #undef DLM_LROWS_H
 #undef DLM_LROWS
         check_launch("latent_attention (rows)");
-        return;
+        if (apart == 0) return 1;
     }
     if (latent_use_mma(dtype, rank, dr, fast)) {
         const int wk = (rank + dr + 63) & ~63, qp = wk + 8;
         const size_t smem = ((size_t)(LM_ROWS + 2 * LA_KC) * qp + 2 * LM_ROWS * LM_PP) * sizeof(__nv_bfloat16) +
                             (2 * LM_ROWS * LA_KC + 3 * LM_ROWS) * sizeof(float);
-        const dim3 grid(T, (H + LM_ROWS - 1) / LM_ROWS, n_splits);
+        const int tokens = rows ? apart : T;
+        const dim3 grid(tokens, (H + LM_ROWS - 1) / LM_ROWS, n_splits);
 #define DLM_LMMA(NT)                                                                                                  \
     do {                                                                                                              \
         auto kern = latent_attention_mma_kernel<NT>;                                                                  \
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
         kern<<<grid, LA_THREADS, smem, stream>>>(q_lat, q_rot, sink, static_cast<const __nv_bfloat16*>(cache),        \
-                                                 block_table, table_width, token_req, positions,                      \
+                                                 block_table, table_width, token_req, positions, rows ? cu_q : nullptr, R, \
                                                  static_cast<__nv_bfloat16*>(lat), partial, T, H, dr, rank, page_size, \
                                                  total_pages, window, scale, n_splits, error_flag_ptr());             \
     } while (0)
@@ -1079,11 +1114,11 @@ void latent_attention(const float* q_lat, const float* q_rot, const float* sink,
 #undef DLM_LMMA
         check_launch("latent_attention (tensor cores)");
         if (n_splits > 1) {
-            launch_dep(latent_merge_kernel<__nv_bfloat16>, dim3(T, H), dim3(128), 0, stream, 
-                partial, n_splits, sink, static_cast<__nv_bfloat16*>(lat), T, H, rank);
+            launch_dep(latent_merge_kernel<__nv_bfloat16>, dim3(tokens, H), dim3(128), 0, stream, 
+                partial, n_splits, sink, rows ? cu_q : nullptr, R, static_cast<__nv_bfloat16*>(lat), T, H, rank);
             check_launch("latent_merge");
         }
-        return;
+        return (rows ? 1 : 0) + (n_splits > 1 ? 2 : 1);
     }
 #define DLM_LAT(TT, NC)                                                                                               \
     launch_latent<TT, NC>(q_lat, q_rot, sink, cache, block_table, table_width, token_req, positions, lat, partial,    \
@@ -1099,6 +1134,7 @@ void latent_attention(const float* q_lat, const float* q_rot, const float* sink,
         else DLM_LAT(__nv_bfloat16, 4);
     }
 #undef DLM_LAT
+    return n_splits > 1 ? 2 : 1;
 }
 
 }  // namespace dlmk
