@@ -407,8 +407,9 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
             bool waited = false;
             for (int it = 0; it < n_tiles; ++it) {
                 const int s = it % NST;
-                // (a stage is given back only after the consumers, who have waited, have read it)
-                if (it >= tiles_before_wait && !waited) { dep_wait(); waited = true; }
+                // (a stage is given back only after the consumers, who wait for the kernel before this one, have read it: that
+                // kernel is not on the clock of the wait for the stage)
+                if ((it >= tiles_before_wait || it >= NST) && !waited) { dep_wait(); waited = true; }
                 if (it >= NST && !mbar_wait(&empty_bar[s], ((it / NST) & 1) ^ 1, abort_flag)) break;
                 const int key0 = keys.at(t_begin + it * BKV);
                 const int lp = key0 >> p.page_shift;

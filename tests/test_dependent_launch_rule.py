@@ -74,6 +74,8 @@ def test_every_wait_on_a_barrier_is_bounded_in_time():
     (body,) = [k[3] for k in KERNELS if k[1] == "gemm_stream_kernel"]
     producer = body[body.index("if (warp == CW)"):]
     assert "dep_wait()" in producer[:producer.index("mbar_wait(&empty_bar")]
+    (body,) = [k[3] for k in KERNELS if k[1] == "attention_decode_tma_kernel"]
+    assert re.search(r"it >= NST\) && !waited\) \{ dep_wait\(\)", body[:body.index("mbar_wait(&empty_bar")])
 
 
 def test_the_setting_belongs_to_a_thread():
