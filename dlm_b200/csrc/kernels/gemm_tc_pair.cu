@@ -15,9 +15,9 @@
 //                       and frees the tensor memory (a joint operation of the pair);
 //   warps 0-7           epilogue of the block's own half (shared with gemm_tc.cu); when a block has drained
 //                       an accumulator, one lane per warp arrives at the leader's "accumulator empty" barrier.
-// No load uses multicast.  Every wait on an mbarrier is bounded, as in gemm_tc.cu; the two blocks meet at
-// cluster barriers after the set-up and before the tensor memory is freed, which every thread of both
-// blocks reaches whatever happened in between.
+// No load uses multicast.  Every wait on an mbarrier is bounded in time, as in gemm_tc.cu; the two blocks meet at
+// cluster barriers after the set-up (which comes after the wait for the kernel before this one) and before the
+// tensor memory is freed, which every thread of both blocks reaches whatever happened in between.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -281,6 +281,7 @@ void launch(const CUtensorMap& mw, const TokenMaps& ma, const TcParams& p, int n
     constexpr int CH = 16;
     constexpr size_t smem = (size_t)STAGES * (W_BYTES + A_ROWS * BK * 2) + EPI_WARPS * CH * 33 * sizeof(float) + 1024;
     static_assert(smem + 1024 <= 227 * 1024, "the ring does not fit in shared memory");
+    static_assert(2 * smem > 227 * 1024, "two blocks of a multiprocessor would wait for one another's tensor memory");
     auto kern = gemm_tc_pair_kernel<STAGES, A_ROWS, CH, EPI, TOut>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int pairs = total_tiles < sm_count() / 2 ? total_tiles : sm_count() / 2;
