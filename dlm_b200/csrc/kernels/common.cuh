@@ -55,19 +55,17 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return t;
 }
 
-// Programmatic dependent launch.  A kernel launched through launch_dep() may be made resident
-// while the kernel before it in the stream is still running, as soon as every block of that kernel
-// has called dep_launch_next() or ended.  It must call dep_wait() before it reads anything an earlier
-// kernel wrote and before it writes anything at all; dep_wait() returns when the earlier kernel
-// has ended and its writes are visible.  (Two exceptions, for data that a kernel before the last one wrote, read past L1: a
-// router's residual, see load_settled in moe_route.cu, and the cache's older keys and values, which the decode attention's TMA
-// copies fetch.)  Every block calls
-// dep_wait() before it ends, so that "this kernel has ended" implies "all earlier kernels have ended".  What a kernel does before
-// dep_wait() (index arithmetic, loads of weights, which no kernel writes) overlaps the end of the
-// kernel before it.  Launched in the ordinary way both calls do nothing.  Pointers to what earlier
-// kernels write (and to what this kernel writes) are not declared __restrict__ in such kernels:
-// the compiler may move an access through a __restrict__ pointer across dep_wait(), which is an
-// assembly statement that clobbers memory and so orders every other access.
+// Programmatic dependent launch.  A kernel launched through launch_dep() may be made resident while the kernel before
+// it in the stream is still running, as soon as every block of that kernel has called dep_launch_next() or ended.  It
+// must call dep_wait() before it reads anything an earlier kernel wrote and before it writes anything at all; dep_wait()
+// returns when the earlier kernel has ended and its writes are visible.  Two exceptions, for data that a kernel before
+// the last one wrote, read past L1: a router's residual (see load_settled in moe_route.cu), and the cache's older keys
+// and values, which the decode attention's TMA copies fetch.  Every block calls dep_wait() before it ends, so that "this
+// kernel has ended" implies "all earlier kernels have ended".  What a kernel does before dep_wait() (index arithmetic,
+// loads of weights, which no kernel writes) overlaps the end of the kernel before it.  Launched in the ordinary way both
+// calls do nothing.  Pointers to what earlier kernels write (and to what this kernel writes) are not declared
+// __restrict__ in such kernels: the compiler may move an access through a __restrict__ pointer across dep_wait(), which
+// is an assembly statement that clobbers memory and so orders every other access.
 __device__ __forceinline__ void dep_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
