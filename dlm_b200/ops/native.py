@@ -34,8 +34,9 @@ class KernelError(RuntimeError):
 
 
 def _longest(batch, tokens: int) -> int:
-    """Tokens of the step's longest request (all the step's, where the batch does not say)."""
-    return int(getattr(batch, "max_q_len", 0)) or tokens
+    """Tokens of the step's longest request; where the batch does not say, what is left if every other brings one (a choice of
+    kernel rests on it, no result does)."""
+    return int(getattr(batch, "max_q_len", 0)) or max(1, tokens - batch.num_requests + 1)
 
 
 class _Branch:
