@@ -134,13 +134,18 @@ router_logits_multi_kernel(const TX* h, const T* __restrict__ w, const float* __
 #pragma unroll
             for (int v = 0; v < ROUTER_WARPS; ++v) part[v] = 0.f;
             for (int base = 0; base < H; base += ROUTER_THREADS) {
+                float val[ROUTER_WARPS];              // all loads in flight before the stores
+#pragma unroll
+                for (int v = 0; v < ROUTER_WARPS; ++v) {
+                    const int i = base + 32 * v + lane;
+                    val[v] = i < H ? to_f32(load_settled(src + i)) : 0.f;
+                }
 #pragma unroll
                 for (int v = 0; v < ROUTER_WARPS; ++v) {
                     const int i = base + 32 * v + lane;
                     if (i < H) {
-                        const float val = to_f32(load_settled(src + i));
-                        x[i] = val;
-                        part[v] = fmaf(val, val, part[v]);
+                        x[i] = val[v];
+                        part[v] = fmaf(val[v], val[v], part[v]);
                     }
                 }
             }
@@ -366,10 +371,19 @@ router_fused_kernel(const TX* h, const T* __restrict__ w, const float* __restric
     float* x = smem;            // [H]
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float ss = 0.f;
-    for (int i = tid; i < H; i += blockDim.x) {
-        const float v = to_f32(load_settled(h + (long long)t * H + i));
-        x[i] = v;
-        ss = fmaf(v, v, ss);
+    for (int i0 = tid; i0 < H; i0 += 8 * ROUTER_THREADS) {      // (eight loads in flight before the stores)
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            v[j] = i0 + j * ROUTER_THREADS < H ? to_f32(load_settled(h + (long long)t * H + i0 + j * ROUTER_THREADS)) : 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int i = i0 + j * ROUTER_THREADS;
+            if (i < H) {
+                x[i] = v[j];
+                ss = fmaf(v[j], v[j], ss);
+            }
+        }
     }
     if (norm_w != nullptr) {
         ss = block_sum(ss, scratch);

@@ -44,9 +44,16 @@ __global__ void streams_expand_kernel(const float* x, float* xs, int S, int H) {
     const int t = blockIdx.x;
     const float* r = x + (long long)t * H;
     float* o = xs + (long long)t * S * H;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) {
-        const float v = r[i];
-        for (int s = 0; s < S; ++s) o[(long long)s * H + i] = v;
+    for (int i0 = threadIdx.x; i0 < H; i0 += 4 * blockDim.x) {      // (four loads in flight before the stores)
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = i0 + j * blockDim.x < H ? r[i0 + j * blockDim.x] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = i0 + j * blockDim.x;
+            if (i < H)
+                for (int s = 0; s < S; ++s) o[(long long)s * H + i] = v[j];
+        }
     }
 }
 
@@ -62,17 +69,36 @@ __global__ void streams_reduce_kernel(const float* xs, const float* __restrict__
     __shared__ float s_part[32];
     const int t = blockIdx.x;
     const float* r = xs + (long long)t * S * H;
-    float part = 0.f;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) {
-        float u = 0.f;
-        for (int s = 0; s < S; ++s) u = fmaf(a ? a[s] : 1.0f, r[(long long)s * H + i], u);
-        su[i] = u;
-        part = fmaf(u, u, part);
-    }
     TOut* o = out + (long long)t * H;
     if (norm_w == nullptr) {
-        for (int i = threadIdx.x; i < H; i += blockDim.x) o[i] = from_f32<TOut>(su[i]);
+        for (int i = threadIdx.x; i < H; i += blockDim.x) {
+            float u = 0.f;
+#pragma unroll 4
+            for (int s = 0; s < S; ++s) u = fmaf(a ? a[s] : 1.0f, r[(long long)s * H + i], u);
+            o[i] = from_f32<TOut>(u);
+        }
         return;
+    }
+    float part = 0.f;
+    for (int i0 = threadIdx.x; i0 < H; i0 += 4 * blockDim.x) {      // (four entries' loads in flight before the stores)
+        float u[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int s = 0; s < S; ++s) {
+            const float w = a ? a[s] : 1.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + j * blockDim.x;
+                if (i < H) u[j] = fmaf(w, r[(long long)s * H + i], u[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = i0 + j * blockDim.x;
+            if (i < H) {
+                su[i] = u[j];
+                part = fmaf(u[j], u[j], part);
+            }
+        }
     }
     const float ss = block_sum(part, s_part);
     const float inv = 1.0f / sqrtf(ss / (float)H + eps);
@@ -89,16 +115,20 @@ __global__ void streams_update_kernel(float* xs, const float* __restrict__ mix, 
     dep_wait();          // nothing is read or written before the kernels before this one have ended
     dep_launch_next();
     __shared__ float s_mix[SC * SC], s_out[SC];
+    const int t = blockIdx.x, first = blockIdx.y * blockDim.x + threadIdx.x;
+    float* r = xs + (long long)t * SC * H;
+    float old[SC], yv = 0.f;                      // (the first column's are on their way while the weights are shared)
+    auto fetch = [&](int i) {
+#pragma unroll
+        for (int s = 0; s < SC; ++s) old[s] = i < H ? r[(long long)s * H + i] : 0.f;
+        if (i < H) yv = y[(long long)t * H + i];
+    };
+    fetch(first);
     for (int i = threadIdx.x; i < SC * SC; i += blockDim.x) s_mix[i] = mix[i];
     for (int i = threadIdx.x; i < SC; i += blockDim.x) s_out[i] = outw[i];
     __syncthreads();
-    const int t = blockIdx.x;
-    float* r = xs + (long long)t * SC * H;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < H; i += gridDim.y * blockDim.x) {
-        float old[SC];
-#pragma unroll
-        for (int s = 0; s < SC; ++s) old[s] = r[(long long)s * H + i];
-        const float yv = y[(long long)t * H + i];
+    for (int i = first; i < H; i += gridDim.y * blockDim.x) {
+        if (i != first) fetch(i);
 #pragma unroll
         for (int d = 0; d < SC; ++d) {
             float v = 0.f;
@@ -119,20 +149,28 @@ __global__ void streams_update_reduce_kernel(float* xs, const float* __restrict_
     dep_launch_next();
     extern __shared__ float su[];        // [H]
     __shared__ float s_mix[SC * SC], s_out[SC], s_in[SC], s_part[32];
+    const int t = blockIdx.x;
+    float* r = xs + (long long)t * SC * H;
+    float next[SC], y_next = 0.f;                 // a column's are on their way while the one before is worked on
+    auto fetch = [&](int i) {
+#pragma unroll
+        for (int s = 0; s < SC; ++s) next[s] = i < H ? r[(long long)s * H + i] : 0.f;
+        if (i < H) y_next = y[(long long)t * H + i];
+    };
+    fetch(threadIdx.x);
     for (int i = threadIdx.x; i < SC * SC; i += blockDim.x) s_mix[i] = mix[i];
     for (int i = threadIdx.x; i < SC; i += blockDim.x) {
         s_out[i] = outw[i];
         s_in[i] = in_next[i];
     }
     __syncthreads();
-    const int t = blockIdx.x;
-    float* r = xs + (long long)t * SC * H;
     float part = 0.f;
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
         float old[SC];
 #pragma unroll
-        for (int s = 0; s < SC; ++s) old[s] = r[(long long)s * H + i];
-        const float yv = y[(long long)t * H + i];
+        for (int s = 0; s < SC; ++s) old[s] = next[s];
+        const float yv = y_next;
+        fetch(i + blockDim.x);                    // (other entries than those that this turn writes)
         float u = 0.f;
 #pragma unroll
         for (int d = 0; d < SC; ++d) {
