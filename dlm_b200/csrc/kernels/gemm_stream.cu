@@ -176,9 +176,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_stream_kernel(StreamParams p)
             for (int pc = 0; pc < passes * p.n_chunks; ++pc, ++it) {
                 const int c = pc % p.n_chunks;
                 const uint32_t s = it % STAGES;
-                // the consumers, who free a stage, wait for the kernel before this one: not on this wait's clock
-                if (it == STAGES && early) dep_wait();
-                if (it >= STAGES && !mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                if (it >= STAGES && !mbar_try_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1)) {
+                    // the consumers, who free a stage, wait for the kernel before this one: not on this wait's clock
+                    if (early) dep_wait();
+                    if (!mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                }
                 const int k0 = c * p.kc;
                 const uint32_t len = (uint32_t)min(p.kc, p.K - k0);
                 if (p.whole_tile) {
@@ -202,9 +204,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_stream_kernel(StreamParams p)
         if (!ok) {
             // copies in flight must land before the block's shared memory is given up; one bound for all of them
             const uint32_t first = it > STAGES ? it - STAGES : 0;
-            uint64_t give_up = 0;
+            const uint64_t give_up = global_ns() + WAIT_LIMIT_NS;
             for (uint32_t j = first; j < it; ++j)
-                if (!mbar_wait_until(&full_bar[j % STAGES], (j / STAGES) & 1, give_up, nullptr)) break;
+                if (!mbar_wait_until(&full_bar[j % STAGES], (j / STAGES) & 1, give_up)) break;
         }
     } else if (warp < CW) {
         // ----------------------------------------------------------------- consumers

@@ -35,27 +35,29 @@ __device__ __forceinline__ uint64_t global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// Waits for the phase until the time `give_up` (0: not set yet; the first wait that needs it sets it, so that several waits
-// can share one), or until `abort_flag` (unless that is null) is set.  The bound is in time: a try may itself block for a
-// while, so a bound in tries could last minutes.  The clock is read once every 16 tries, which a wait that is met in time
-// hardly ever reaches.
-__device__ __forceinline__ bool mbar_wait_until(uint64_t* bar, uint32_t parity, uint64_t& give_up, volatile int* abort_flag) {
-    for (uint32_t i = 0;; ++i) {
+// Bounded wait of a role.  Returns false when it gave up (or another role already had): the caller stops.  The bound is in time
+// (a try may itself block for a while, so a bound in tries could last minutes); the clock is read once every 16 tries,
+// which a wait that is met in time hardly ever reaches.  (The loop's own end lies far beyond the time: without one the compiled
+// loop costs the streaming product of a few rows 2 %.)
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    uint64_t give_up = 0;
+    for (uint32_t i = 0; i < 1u << 30; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
-        if (abort_flag != nullptr && *abort_flag) return false;
+        if (*abort_flag) return false;
         if ((i & 15) == 15) {
             const uint64_t now = global_ns();
             if (give_up == 0) give_up = now + WAIT_LIMIT_NS;
-            else if (now > give_up) return false;
+            else if (now > give_up) break;
         }
     }
-}
-// Bounded wait of a role.  Returns false when it gave up (or another role already had): the caller stops.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    uint64_t give_up = 0;
-    if (mbar_wait_until(bar, parity, give_up, abort_flag)) return true;
     *abort_flag = 1;
     return false;
+}
+// Waits for the phase until the time `give_up`, which several waits may share.
+__device__ __forceinline__ bool mbar_wait_until(uint64_t* bar, uint32_t parity, uint64_t give_up) {
+    while (!mbar_try_wait(bar, parity))
+        if (global_ns() > give_up) return false;
+    return true;
 }
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
